@@ -143,27 +143,35 @@ struct DeviceTables {
 static std::mutex g_dev_mtx;
 static DeviceTables g_dev[64];
 
+template <class K>
+static void set_smem(K* kernel, int bytes) {
+  CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+}
+
+template <int N, int PLAN>
+static void set_z_attrs() {
+  set_smem(k_zinv<N, 8, 1, PLAN>, ZCfg<N, 8>::SMEM);
+  set_smem(k_zinv<N, 32, 1, PLAN>, ZCfg<N, 32>::SMEM);
+  set_smem(k_zinv<N, 32, 8, PLAN>, ZCfg<N, 32>::SMEM);
+  set_smem(k_zfwd<N, 8, 1, PLAN>, ZCfg<N, 8>::SMEM);
+  set_smem(k_zfwd<N, 32, 1, PLAN>, ZCfg<N, 32>::SMEM);
+  set_smem(k_zfwd<N, 32, 8, PLAN>, ZCfg<N, 32>::SMEM);
+}
+
+// Lengths with two radix plans (fft_smem PLAN).
+__host__ __device__ constexpr bool two_plans(int n) { return n == 64 || n == 128 || n == 256; }
+
 template <int N, class C>
 static void set_pass_attrs() {
   const int bytes = N * (TILE_LINES + 1) * (int)sizeof(C);
-  CK(cudaFuncSetAttribute(k_pass<N, -1, PRO_LOAD, EPI_STORE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-  CK(cudaFuncSetAttribute(k_pass<N, +1, PRO_LOAD, EPI_STORE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  set_smem(k_pass<N, -1, C>, bytes);
+  set_smem(k_pass<N, +1, C>, bytes);
   if constexpr (sizeof(C) == 8) {
-    CK(cudaFuncSetAttribute(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    CK(cudaFuncSetAttribute(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    CK(cudaFuncSetAttribute(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    CK(cudaFuncSetAttribute(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    CK(cudaFuncSetAttribute(k_xline<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if constexpr (N == 64 || N == 128 || N == 256) {  // the alternative radix plan (fft_smem PLAN 1)
-      CK(cudaFuncSetAttribute(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C, 1, 1>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      CK(cudaFuncSetAttribute(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C, 1, 1>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      CK(cudaFuncSetAttribute(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C, 8, 1>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      CK(cudaFuncSetAttribute(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C, 8, 1>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-      CK(cudaFuncSetAttribute(k_xline<N, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+    set_smem(k_xline<N>, bytes);
+    if constexpr (N <= 256) set_z_attrs<N, 0>();
+    if constexpr (two_plans(N)) {
+      set_z_attrs<N, 1>();
+      set_smem(k_xline<N, 1>, bytes);
     }
   }
 }
@@ -255,59 +263,30 @@ static cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t st) {
   return cudaMallocFromPoolAsync(p, bytes, device_tables(dev).pool, st);
 }
 
-// ---------------------------------------------------------------- pass launcher
+// ---------------------------------------------------------------- pass launchers
 template <int N, class C>
-static void launch_pass_n(int dir, int pro, int epi, const PassArgs& a, const DevVolume& v, const DevChains& ch,
-                          const C* tw, int nch, cudaStream_t s) {
-  const dim3 grid(cdiv_i((long long)a.A * a.B, TILE_LINES), a.chain_only >= 0 ? 1 : nch);
-  const dim3 block(PassCfg<N>::NT);
+static void launch_pass_n(int dir, const PassArgs& a, const DevChains& ch, const C* tw, int nch, cudaStream_t s) {
+  const dim3 grid(cdiv_i((long long)a.A * a.B, TILE_LINES), nch);
   const size_t smem = (size_t)N * (TILE_LINES + 1) * sizeof(C);
-  if (dir < 0 && pro == PRO_LOAD && epi == EPI_STORE)
-    launch_k(k_pass<N, -1, PRO_LOAD, EPI_STORE, C>, grid, block, smem, s, a, v, ch, tw);
-  else if (dir > 0 && pro == PRO_LOAD && epi == EPI_STORE)
-    launch_k(k_pass<N, +1, PRO_LOAD, EPI_STORE, C>, grid, block, smem, s, a, v, ch, tw);
-  else if constexpr (sizeof(C) == 8) {
-    // the z passes touch the chain-minor arrays: with 8 or more chains, tiles of 4 lines x 8 chains unless the chain
-    // set's tuning chose tiles of 32 lines of one chain (ch.ztile)
-    const bool grouped = a.chain_only < 0 && nch >= 8 && a.B > 1 && ch.ztile != 1;
-    const dim3 ggrid(cdiv_i((long long)a.A * a.B, TILE_LINES / 8), cdiv_i(nch, 8));
-    // the radix plan the chain set's tuning chose (ch.fftplan) for the lengths that have two
-    constexpr bool two_plans = N == 64 || N == 128 || N == 256;
-    const bool alt = two_plans && (ch.fftplan & (dir > 0 ? FP_ZINV : FP_ZFWD)) != 0;
-    if (dir > 0 && pro == PRO_DATAGRAD && epi == EPI_STORE) {
-      if (alt && grouped) launch_k(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C, 8, 1>, ggrid, block, smem, s, a, v, ch, tw);
-      else if (alt) launch_k(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C, 1, 1>, grid, block, smem, s, a, v, ch, tw);
-      else if (grouped) launch_k(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C, 8>, ggrid, block, smem, s, a, v, ch, tw);
-      else launch_k(k_pass<N, +1, PRO_DATAGRAD, EPI_STORE, C>, grid, block, smem, s, a, v, ch, tw);
-    } else if (dir < 0 && pro == PRO_LOAD && epi == EPI_GATHER) {
-      if (alt && grouped) launch_k(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C, 8, 1>, ggrid, block, smem, s, a, v, ch, tw);
-      else if (alt) launch_k(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C, 1, 1>, grid, block, smem, s, a, v, ch, tw);
-      else if (grouped) launch_k(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C, 8>, ggrid, block, smem, s, a, v, ch, tw);
-      else launch_k(k_pass<N, -1, PRO_LOAD, EPI_GATHER, C>, grid, block, smem, s, a, v, ch, tw);
-    } else {
-      throw Error(DR_ERR_INVALID, "unsupported pass combination");
-    }
-  } else {
-    throw Error(DR_ERR_INVALID, "unsupported pass combination");
-  }
+  if (dir < 0) launch_k(k_pass<N, -1, C>, grid, PassCfg<N>::NT, smem, s, a, ch, tw);
+  else launch_k(k_pass<N, +1, C>, grid, PassCfg<N>::NT, smem, s, a, ch, tw);
   CK_LAUNCH();
 }
 
 template <class C>
-static void launch_pass(int n, int dir, int pro, int epi, const PassArgs& a, const DevVolume& v, const DevChains& ch,
-                        const C* tw, int nch, cudaStream_t s) {
+static void launch_pass(int n, int dir, const PassArgs& a, const DevChains& ch, const C* tw, int nch, cudaStream_t s) {
   switch (n) {
-    case 2: launch_pass_n<2, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
-    case 4: launch_pass_n<4, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
-    case 8: launch_pass_n<8, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
-    case 16: launch_pass_n<16, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
-    case 32: launch_pass_n<32, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
-    case 64: launch_pass_n<64, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
-    case 128: launch_pass_n<128, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
-    case 256: launch_pass_n<256, C>(dir, pro, epi, a, v, ch, tw, nch, s); break;
+    case 2: launch_pass_n<2, C>(dir, a, ch, tw, nch, s); break;
+    case 4: launch_pass_n<4, C>(dir, a, ch, tw, nch, s); break;
+    case 8: launch_pass_n<8, C>(dir, a, ch, tw, nch, s); break;
+    case 16: launch_pass_n<16, C>(dir, a, ch, tw, nch, s); break;
+    case 32: launch_pass_n<32, C>(dir, a, ch, tw, nch, s); break;
+    case 64: launch_pass_n<64, C>(dir, a, ch, tw, nch, s); break;
+    case 128: launch_pass_n<128, C>(dir, a, ch, tw, nch, s); break;
+    case 256: launch_pass_n<256, C>(dir, a, ch, tw, nch, s); break;
     case 512:
       if constexpr (sizeof(C) == 8) {
-        launch_pass_n<512, C>(dir, pro, epi, a, v, ch, tw, nch, s);
+        launch_pass_n<512, C>(dir, a, ch, tw, nch, s);
         break;
       }
       [[fallthrough]];
@@ -316,29 +295,66 @@ static void launch_pass(int n, int dir, int pro, int epi, const PassArgs& a, con
 }
 
 static PassArgs pass_args(const void* in, void* out, long long in_cs, long long out_cs, int A, int B, int n_in,
-                          int n_out, double scale = 1.0, int step = -1, int sel = 0, int write_o = 0,
-                          int chain_only = -1) {
+                          int n_out, int step = -1) {
   PassArgs a;
   a.in = in; a.out = out; a.in_cs = in_cs; a.out_cs = out_cs;
-  a.A = A; a.B = B; a.n_in = n_in; a.n_out = n_out; a.scale = scale;
-  a.step = step; a.sel = sel; a.write_o = write_o; a.chain_only = chain_only;
+  a.A = A; a.B = B; a.n_in = n_in; a.n_out = n_out;
+  a.step = step;
   return a;
 }
 
-// Unpruned in-place 3D FFT of one (or nch chain-strided) field(s).
-template <class C>
-static void fft3d(C* f, const int* E, int dir, long long cs, int nch, const C* tw, cudaStream_t s,
-                  const DevVolume& v, const DevChains& ch, int chain_only = -1) {
-  const int E0 = E[0], E1 = E[1], E2 = E[2];
-  if (dir < 0) {
-    launch_pass<C>(E0, -1, PRO_LOAD, EPI_STORE, pass_args(f, f, cs, cs, E1 * E2, 1, E0, E0, 1.0, -1, 0, 0, chain_only), v, ch, tw, nch, s);
-    launch_pass<C>(E1, -1, PRO_LOAD, EPI_STORE, pass_args(f, f, cs, cs, E2, E0, E1, E1, 1.0, -1, 0, 0, chain_only), v, ch, tw, nch, s);
-    launch_pass<C>(E2, -1, PRO_LOAD, EPI_STORE, pass_args(f, f, cs, cs, 1, E0 * E1, E2, E2, 1.0, -1, 0, 0, chain_only), v, ch, tw, nch, s);
-  } else {
-    launch_pass<C>(E0, +1, PRO_LOAD, EPI_STORE, pass_args(f, f, cs, cs, E1 * E2, 1, E0, E0, 1.0, -1, 0, 0, chain_only), v, ch, tw, nch, s);
-    launch_pass<C>(E1, +1, PRO_LOAD, EPI_STORE, pass_args(f, f, cs, cs, E2, E0, E1, E1, 1.0, -1, 0, 0, chain_only), v, ch, tw, nch, s);
-    launch_pass<C>(E2, +1, PRO_LOAD, EPI_STORE, pass_args(f, f, cs, cs, 1, E0 * E1, E2, E2, 1.0, -1, 0, 0, chain_only), v, ch, tw, nch, s);
+template <int N, int TL, int CPB, int PLAN>
+static void launch_z_t(int dir, const ZArgs& a, const DevVolume& v, const DevChains& ch, const float2* tw, cudaStream_t s) {
+  const dim3 grid(cdiv_i((long long)v.by * v.bx / 2, TL / CPB), cdiv_i(ch.C, CPB));
+  if (dir > 0) launch_k(k_zinv<N, TL, CPB, PLAN>, grid, ZCfg<N, TL>::NT, ZCfg<N, TL>::SMEM, s, a, v, ch, tw);
+  else launch_k(k_zfwd<N, TL, CPB, PLAN>, grid, ZCfg<N, TL>::NT, ZCfg<N, TL>::SMEM, s, a, v, ch, tw);
+  CK_LAUNCH();
+}
+
+// The tile of a z pass: with 8 or more chains 4 pair lines x 8 chains unless the chain set's tuning chose tiles of one
+// chain (ch.ztile); those hold 32 pair lines, or 8 while 32 would give fewer than two blocks per SM.
+template <int N, int PLAN>
+static void launch_z_n(int dir, const ZArgs& a, const DevVolume& v, const DevChains& ch, const float2* tw, cudaStream_t s) {
+  if (ch.C >= 8 && ch.ztile != 1) launch_z_t<N, 32, 8, PLAN>(dir, a, v, ch, tw, s);
+  else if ((long long)cdiv_i((long long)v.by * v.bx / 2, 32) * ch.C >= 296) launch_z_t<N, 32, 1, PLAN>(dir, a, v, ch, tw, s);
+  else launch_z_t<N, 8, 1, PLAN>(dir, a, v, ch, tw, s);
+}
+
+template <int N>
+static void launch_z_plan(int dir, const ZArgs& a, const DevVolume& v, const DevChains& ch, const float2* tw, cudaStream_t s) {
+  if constexpr (two_plans(N)) {
+    if (ch.fftplan & (dir > 0 ? FP_ZINV : FP_ZFWD)) return launch_z_n<N, 1>(dir, a, v, ch, tw, s);
   }
+  launch_z_n<N, 0>(dir, a, v, ch, tw, s);
+}
+
+// The z pass of every chain: dir > 0 gD -> T2, dir < 0 T2 -> mu_D (and mu_O).
+static void launch_z(int dir, const ZArgs& a, const DevVolume& v, const DevChains& ch, const float2* tw, cudaStream_t s) {
+  switch (v.E2) {
+    case 2: launch_z_plan<2>(dir, a, v, ch, tw, s); break;
+    case 4: launch_z_plan<4>(dir, a, v, ch, tw, s); break;
+    case 8: launch_z_plan<8>(dir, a, v, ch, tw, s); break;
+    case 16: launch_z_plan<16>(dir, a, v, ch, tw, s); break;
+    case 32: launch_z_plan<32>(dir, a, v, ch, tw, s); break;
+    case 64: launch_z_plan<64>(dir, a, v, ch, tw, s); break;
+    case 128: launch_z_plan<128>(dir, a, v, ch, tw, s); break;
+    case 256: launch_z_plan<256>(dir, a, v, ch, tw, s); break;
+    default: throw Error(DR_ERR_UNSUPPORTED, "FFT length not supported: " + std::to_string(v.E2));
+  }
+}
+static ZArgs zinv_args(int step = -1) { return ZArgs{step, 0, 0, 1.0f}; }
+static ZArgs zfwd_args(const DevVolume& v, int step, int sel, int write_o) {
+  return ZArgs{step, sel, write_o, (float)(1.0 / (double)v.N)};
+}
+
+// Unpruned in-place 3D FFT of one field.
+template <class C>
+static void fft3d(C* f, const int* E, int dir, const C* tw, cudaStream_t s) {
+  const int E0 = E[0], E1 = E[1], E2 = E[2];
+  const DevChains none{};
+  launch_pass<C>(E0, dir, pass_args(f, f, 0, 0, E1 * E2, 1, E0, E0), none, tw, 1, s);
+  launch_pass<C>(E1, dir, pass_args(f, f, 0, 0, E2, E0, E1, E1), none, tw, 1, s);
+  launch_pass<C>(E2, dir, pass_args(f, f, 0, 0, 1, E0 * E1, E2, E2), none, tw, 1, s);
 }
 
 // ---------------------------------------------------------------- volume
@@ -641,6 +657,8 @@ static void volume_build_device(Volume* V, const float* covariance, int covfun, 
   DevVolume& dv = V->dv;
   cudaStream_t st = V->stream;
   dv.E0 = hv.E[0]; dv.E1 = hv.E[1]; dv.E2 = hv.E[2]; dv.N = hv.N;
+  dv.EZ = dv.E2 / 2 + 1;
+  dv.NH = (long long)dv.EZ * dv.E1 * dv.E0;
   dv.bx = hv.box[0]; dv.by = hv.box[1]; dv.bz = hv.box[2];
   dv.n_h = (int)hv.Yh.size(); dv.n_s = (int)hv.Ys.size(); dv.n_o = (int)hv.o_flat.size();
   dv.box_to_d = V->upload(hv.box_to_d);
@@ -675,9 +693,8 @@ static void volume_build_device(Volume* V, const float* covariance, int covfun, 
                                            Q[9], Q[10], (double)covariance[0], (double)covariance[1],
                                            (double)covariance[2], covfun);
     CK_LAUNCH();
-    DevChains none{};
-    fft3d<double2>(base, hv.E, -1, 0, 1, V->tw_d, st, dv, none);
-    k_spectrum<<<cdiv_i(N, 256), 256, 0, st>>>(base, sinv, V->lam_re, N, nS);
+    fft3d<double2>(base, hv.E, -1, V->tw_d, st);
+    k_spectrum<<<cdiv_i(N, 256), 256, 0, st>>>(base, sinv, V->lam_re, hv.E[0], hv.E[1], hv.E[2], nS);
     CK_LAUNCH();
     double2 l0;
     CK(cudaMemcpyAsync(&l0, base, sizeof(double2), cudaMemcpyDeviceToHost, st));
@@ -882,9 +899,9 @@ static int l2_prefetch_flag() {
 static void launch_xline(Chainset* S, int step, int flags) {
   flags |= l2_prefetch_flag();
   const DevVolume& v = S->vol->dv;
-  if (cdiv_i((long long)v.E1 * v.E2, TILE_LINES) > S->dc.maxblk)
+  if (cdiv_i((long long)v.E1 * v.EZ, TILE_LINES) > S->dc.maxblk)
     throw Error(DR_ERR_STATE, "partial-sum buffer smaller than the x-line block count");
-  const dim3 grid(cdiv_i((long long)v.E1 * v.E2, TILE_LINES), S->C);
+  const dim3 grid(cdiv_i((long long)v.E1 * v.EZ, TILE_LINES), S->C);
   const size_t smem = (size_t)v.E0 * (TILE_LINES + 1) * sizeof(float2);
   const float2* tw = S->vol->tw_f;
   switch (v.E0) {
@@ -915,7 +932,7 @@ template <int E, bool PF>
 static void launch_plane_t(Chainset* S, int step, int flags) {
   flags |= l2_prefetch_flag();
   const DevVolume& v = S->vol->dv;
-  const dim3 grid(v.E2, S->C);
+  const dim3 grid(v.EZ, S->C);
   const size_t smem = (size_t)plane_layout(E, PlaneGeom<E>::SIZE, PF).total;
   launch_k(k_xyplane<E, PF>, grid, PlaneCfg<E, PF>::NT, smem, S->stream, v, S->dc, step, flags, S->vol->tw_f);
   CK_LAUNCH();
@@ -923,7 +940,7 @@ static void launch_plane_t(Chainset* S, int step, int flags) {
 
 static void launch_plane(Chainset* S, int step, int flags) {
   const DevVolume& v = S->vol->dv;
-  if (v.E2 > S->dc.maxblk) throw Error(DR_ERR_STATE, "partial-sum buffer smaller than the plane count");
+  if (v.EZ > S->dc.maxblk) throw Error(DR_ERR_STATE, "partial-sum buffer smaller than the plane count");
   if (S->tma) {
     switch (v.E0) {
       case 4: launch_plane_t<4, true>(S, step, flags); return;
@@ -945,39 +962,50 @@ static void launch_plane(Chainset* S, int step, int flags) {
   }
 }
 
+// The momentum of an iteration and the trajectory of Im mu (k_momentum); with XF_FIXED_MOMENTUM from Gq.
+static void launch_momentum(Chainset* S, int flags) {
+  const DevVolume& v = S->vol->dv;
+  const dim3 grid(S->dc.nb_g, S->C);
+  if (flags & XF_FIXED_MOMENTUM) launch_k(k_momentum<true>, grid, MOM_NT, 0, S->stream, v, S->dc);
+  else launch_k(k_momentum<false>, grid, MOM_NT, 0, S->stream, v, S->dc);
+  CK_LAUNCH();
+}
+
+// The y passes of the x-line path.
+static void launch_y(Chainset* S, int dir, int step) {
+  const DevVolume& v = S->vol->dv;
+  const DevChains& ch = S->dc;
+  if (dir < 0)
+    launch_pass<float2>(v.E1, -1, pass_args(ch.T1, ch.T2, ch.t1_stride, ch.t2_stride, v.EZ, v.bx, v.E1, v.by, step), ch,
+                        S->vol->tw_f, S->C, S->stream);
+  else
+    launch_pass<float2>(v.E1, +1, pass_args(ch.T2, ch.T1, ch.t2_stride, ch.t1_stride, v.EZ, v.bx, v.by, v.E1, step), ch,
+                        S->vol->tw_f, S->C, S->stream);
+}
+
 // The gradient/leapfrog sequence for steps 0..L (see kernels.cu header).
 static void enqueue_steps(Chainset* S, int L, int flags) {
   const DevVolume& v = S->vol->dv;
   const DevChains& ch = S->dc;
   const float2* tw = S->vol->tw_f;
-  const int C = S->C;
+  launch_momentum(S, flags);
   for (int s = 0; s <= L; s++) {
-    const NvtxRange range(s == 0 ? "leapfrog step 0 (momentum, half kick, drift)"
+    const NvtxRange range(s == 0 ? "leapfrog step 0 (half kick, drift)"
                                  : (s == L ? "leapfrog last step (half kick, energies)" : "leapfrog step"));
     const int sel = s == 0 ? 0 : 1;
     if (s > 0) {
-      if (!S->plane)
-        launch_pass<float2>(v.E1, -1, PRO_LOAD, EPI_STORE,
-                            pass_args(ch.T1, ch.T2, ch.t1_stride, ch.t2_stride, v.E2, v.bx, v.E1, v.by, 1.0, s), v, ch,
-                            tw, C, S->stream);
+      if (!S->plane) launch_y(S, -1, s);
       // forward z (pruned to the box), gather mu at data / output voxels
-      launch_pass<float2>(v.E2, -1, PRO_LOAD, EPI_GATHER,
-                          pass_args(ch.T2, nullptr, ch.t2_stride, 0, 1, v.by * v.bx, v.E2, v.bz,
-                                    1.0 / (double)v.N, s, 1, 2),
-                          v, ch, tw, C, S->stream);
+      launch_z(-1, zfwd_args(v, s, 1, 2), v, ch, tw, S->stream);
     }
     if (v.n_s > 0) launch_spmv(S, s, sel, -1, true);
     launch_spmv(S, s, sel, -1, false);
     // inverse z from the box back to spectral z
-    launch_pass<float2>(v.E2, +1, PRO_DATAGRAD, EPI_STORE,
-                        pass_args(nullptr, ch.T2, 0, ch.t2_stride, 1, v.by * v.bx, v.bz, v.E2, 1.0, s), v, ch, tw, C,
-                        S->stream);
+    launch_z(+1, zinv_args(s), v, ch, tw, S->stream);
     if (S->plane) {
       launch_plane(S, s, flags);
     } else {
-      launch_pass<float2>(v.E1, +1, PRO_LOAD, EPI_STORE,
-                          pass_args(ch.T2, ch.T1, ch.t2_stride, ch.t1_stride, v.E2, v.bx, v.by, v.E1, 1.0, s), v, ch,
-                          tw, C, S->stream);
+      launch_y(S, +1, s);
       launch_xline(S, s, flags);
     }
   }
@@ -1294,7 +1322,6 @@ static TuneChoice autotune(Volume* V, int C, const dr_hmc_opts* o) {
     }
     // the second radix plan, one transform at a time on the best configuration so far: the inverse and the forward
     // z passes, and the x transforms of the x-line kernel, where their length has two plans
-    auto two_plans = [](int n) { return n == 64 || n == 128 || n == 256; };
     for (int bit : {(int)FP_ZINV, (int)FP_ZFWD, (int)FP_XLINE}) {
       if (bit == FP_XLINE ? !(best.path == 2 && two_plans(v.E0)) : !two_plans(v.E2)) continue;
       TuneChoice t = best;
@@ -1342,7 +1369,7 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   if (S->NR > 8) throw Error(DR_ERR_UNSUPPORTED, "too many chains");
   if (S->NR == 3) S->NR = 4;
   if (S->NR > 4 && S->NR < 8) S->NR = 8;
-  const long long N = v.N;
+  const long long N = v.N, NH = v.NH;
   const PathOptions po = path_options(v, V->device);
   int path = po.plane ? 0 : 2, grid = 8;
   // tensor-core products by default for 32 or more chains; the tuner, DRB_TC_PRODUCTS=0 / 1 and a forced choice
@@ -1378,19 +1405,21 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   if ((path == 0 && !po.plane) || (path == 1 && !po.prefetch)) path = po.plane ? 0 : 2;
   // the state arrays are allocated after the tuning, whose candidate chain sets then reuse the pool's memory
   // without this chain set's arrays held beside them
-  ch.U = S->alloc<float2>((size_t)C * 2 * N);
-  ch.Q = S->alloc<float2>((size_t)C * N);
+  ch.U = S->alloc<float2>((size_t)C * 2 * NH);
+  ch.G = S->alloc<float2>((size_t)C * 2 * NH);
+  ch.Q = S->alloc<float2>((size_t)C * NH);
+  ch.Gq = S->alloc<float2>(NH);
   S->path = path;
   S->grid = grid;
   S->plane = path != 2;
   S->tma = path == 1;
-  ch.t2_stride = (long long)v.E2 * v.by * v.bx;
+  ch.t2_stride = (long long)v.EZ * v.by * v.bx;
   if (S->plane) {
     // T1 is only needed by the initial transforms: borrow the momentum buffer
-    ch.t1_stride = N;
+    ch.t1_stride = NH;
     ch.T1 = ch.Q;
   } else {
-    ch.t1_stride = (long long)v.E2 * v.E1 * v.bx;
+    ch.t1_stride = (long long)v.EZ * v.E1 * v.bx;
     ch.T1 = S->alloc<float2>((size_t)C * ch.t1_stride);
   }
   ch.T2 = S->alloc<float2>((size_t)C * ch.t2_stride);
@@ -1398,7 +1427,7 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   ch.muO = S->alloc<float>((size_t)2 * std::max(v.n_o, 1) * C);
   ch.gD = S->alloc<float>((size_t)v.n_h * C);
   ch.rs = S->alloc<float>((size_t)std::max(v.n_s, 1) * C);
-  ch.nb_x = S->plane ? v.E2 : cdiv_i((long long)v.E1 * v.E2, TILE_LINES);
+  ch.nb_x = S->plane ? v.EZ : cdiv_i((long long)v.E1 * v.EZ, TILE_LINES);
   const int wide = device_tables(V->device).sms * S->grid;
   ch.nb_w = std::max(1, std::min(v.n_s, wide));
   ch.nb_wt = std::max(1, std::min(cdiv_i(v.n_h, 8), wide));
@@ -1411,7 +1440,9 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
     const char* tg = std::getenv("DRB_TC_TMA_GATHER");
     S->tc_tg = !(tg && std::string(tg) == "0") && encode_row_map(&S->tc_map_wt, ch.rs, ch.Cp, (long long)v.n_s, S->tc_N);
   }
-  ch.maxblk = std::max(ch.nb_x, std::max(ch.nb_w, ch.nb_wt));
+  // k_momentum's row groups, at most four blocks per SM taking them in turn
+  ch.nb_g = std::min(cdiv_i((long long)v.EZ * v.E1, MOM_ITEMS / v.E0), 592);
+  ch.maxblk = std::max(ch.nb_x + ch.nb_g, std::max(ch.nb_w, ch.nb_wt));
   ch.part = S->alloc<double>((size_t)C * NSLOT * ch.maxblk);
   ch.st = S->alloc<ChainState>(C);
   ch.s1 = S->alloc<double>((size_t)std::max(v.n_o, 1) * C);
@@ -1434,14 +1465,14 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   CK_LAUNCH();
   k_fill_gD<<<std::max(1, cdiv_i((long long)v.n_h * C, 256)), 256, 0, s>>>(v, ch);
   CK_LAUNCH();
-  launch_pass<float2>(v.E2, +1, PRO_DATAGRAD, EPI_STORE, pass_args(nullptr, ch.T2, 0, ch.t2_stride, 1, v.by * v.bx, v.bz, v.E2), v, ch, tw, C, s);
-  launch_pass<float2>(v.E1, +1, PRO_LOAD, EPI_STORE, pass_args(ch.T2, ch.T1, ch.t2_stride, ch.t1_stride, v.E2, v.bx, v.by, v.E1), v, ch, tw, C, s);
-  launch_pass<float2>(v.E0, +1, PRO_LOAD, EPI_STORE, pass_args(ch.T1, ch.U, ch.t1_stride, 2 * N, v.E2 * v.E1, 1, v.bx, v.E0), v, ch, tw, C, s);
-  k_init_prior<<<dim3(std::max(1, cdiv_i(N / 2, 256)), C), 256, 0, s>>>(v, ch);
+  launch_z(+1, zinv_args(), v, ch, tw, s);
+  launch_y(S, +1, -1);
+  launch_pass<float2>(v.E0, +1, pass_args(ch.T1, ch.U, ch.t1_stride, 2 * NH, v.EZ * v.E1, 1, v.bx, v.E0), ch, tw, C, s);
+  k_init_prior<<<dim3(cdiv_i(NH, 256), C), 256, 0, s>>>(v, ch);
   CK_LAUNCH();
-  launch_pass<float2>(v.E0, -1, PRO_LOAD, EPI_STORE, pass_args(ch.U, ch.T1, 2 * N, ch.t1_stride, v.E2 * v.E1, 1, v.E0, v.bx), v, ch, tw, C, s);
-  launch_pass<float2>(v.E1, -1, PRO_LOAD, EPI_STORE, pass_args(ch.T1, ch.T2, ch.t1_stride, ch.t2_stride, v.E2, v.bx, v.E1, v.by), v, ch, tw, C, s);
-  launch_pass<float2>(v.E2, -1, PRO_LOAD, EPI_GATHER, pass_args(ch.T2, nullptr, ch.t2_stride, 0, 1, v.by * v.bx, v.E2, v.bz, 1.0 / (double)N, -1, 0, 1), v, ch, tw, C, s);
+  launch_pass<float2>(v.E0, -1, pass_args(ch.U, ch.T1, 2 * NH, ch.t1_stride, v.EZ * v.E1, 1, v.E0, v.bx), ch, tw, C, s);
+  launch_y(S, -1, -1);
+  launch_z(-1, zfwd_args(v, -1, 0, 1), v, ch, tw, s);
   CK(cudaStreamSynchronize(s));
 }
 
@@ -1563,6 +1594,32 @@ static void upload_field(Chainset* S, const float* mu) {
   CK(cudaMemcpyAsync(S->tmp, mu, sizeof(float2) * S->vol->dv.N, cudaMemcpyHostToDevice, S->stream));
 }
 
+// A complex field's spectrum (S->tmp, N modes) into half spectra of its real and imaginary parts, and back.
+static void split_spectrum(Chainset* S, float2* h, float2* g) {
+  const DevVolume& v = S->vol->dv;
+  k_split<<<cdiv_i(v.NH, 256), 256, 0, S->stream>>>(v, S->tmp, h, g);
+  CK_LAUNCH();
+}
+// u = IFFT of the field in S->tmp as the half spectra h and g.
+static void forward_field(Chainset* S, float2* h, float2* g) {
+  fft3d<float2>(S->tmp, S->vol->hv.E, +1, S->vol->tw_f, S->stream);
+  split_spectrum(S, h, g);
+}
+// The real-space field of the half spectra h and g into host memory (2N floats).
+static void download_field(Chainset* S, const float2* h, const float2* g, float* out) {
+  const DevVolume& v = S->vol->dv;
+  k_merge<<<cdiv_i(v.N, 256), 256, 0, S->stream>>>(v, h, g, S->tmp);
+  CK_LAUNCH();
+  fft3d<float2>(S->tmp, S->vol->hv.E, -1, S->vol->tw_f, S->stream);
+  k_scale<<<cdiv_i(v.N, 256), 256, 0, S->stream>>>(S->tmp, v.N, 1.0f / (float)v.N);
+  CK_LAUNCH();
+  CK(cudaMemcpyAsync(out, S->tmp, sizeof(float2) * v.N, cudaMemcpyDeviceToHost, S->stream));
+}
+// Offset of a chain's accepted (half = acc) or proposal state in U and G.
+static long long state_off(const Chainset* S, int chain, int half) {
+  return ((long long)chain * 2 + half) * S->vol->dv.NH;
+}
+
 static void gather_data(Chainset* S, const float2* field, int c, int half, bool with_output) {
   const DevVolume& v = S->vol->dv;
   k_gather_re<<<cdiv_i(v.n_h, 256), 256, 0, S->stream>>>(field, v.d_flat, v.n_h, S->dc.muD + (long long)half * v.n_h * S->C, S->C, c, v.N, S->dc.err);
@@ -1597,13 +1654,11 @@ static void eval_sampler(Chainset* S, int chain, const float* mu, double* lpll, 
   read_states(S, &st);
   saved = st;
   const int half = st[chain].acc ^ 1;
-  DevChains none{};
   upload_field(S, mu);
   gather_data(S, S->tmp, chain, half, false);
-  fft3d<float2>(S->tmp, S->vol->hv.E, +1, 0, 1, S->vol->tw_f, S->stream, v, none);
-  CK(cudaMemcpyAsync(S->dc.U + ((long long)chain * 2 + half) * v.N, S->tmp, sizeof(float2) * v.N,
-                     cudaMemcpyDeviceToDevice, S->stream));
-  CK(cudaMemsetAsync(S->dc.Q + (long long)chain * v.N, 0, sizeof(float2) * v.N, S->stream));
+  forward_field(S, S->dc.U + state_off(S, chain, half), S->dc.G + state_off(S, chain, half));
+  CK(cudaMemsetAsync(S->dc.Q + (long long)chain * v.NH, 0, sizeof(float2) * v.NH, S->stream));
+  CK(cudaMemsetAsync(S->dc.Gq, 0, sizeof(float2) * v.NH, S->stream));
   for (int c = 0; c < S->C; c++) st[c].L_cur = -1;
   st[chain].L_cur = 0;
   st[chain].eps_cur = 2.0f;
@@ -1612,20 +1667,13 @@ static void eval_sampler(Chainset* S, int chain, const float* mu, double* lpll, 
   try {
     enqueue_steps(S, 0, XF_FIXED_MOMENTUM | XF_WRITE_Q_LAST);
     if (lpll) {
-      const double lp = part_sum(S, chain, SL_LP0, S->dc.nb_x);
+      const double lp = part_sum(S, chain, SL_LP0, S->dc.nb_x + S->dc.nb_g);
       const double Rh = part_sum(S, chain, SL_RH0, S->dc.nb_wt);
       const double Rs = v.n_s > 0 ? part_sum(S, chain, SL_RS0, S->dc.nb_w) : 0.0;
       lpll[0] = -0.5 * lp / (double)v.N;
       lpll[1] = -0.5 * ((double)st[chain].sh * Rh + (v.n_s > 0 ? (double)st[chain].ss * Rs : 0.0));
     }
-    if (grad) {
-      CK(cudaMemcpyAsync(S->tmp, S->dc.Q + (long long)chain * v.N, sizeof(float2) * v.N, cudaMemcpyDeviceToDevice,
-                         S->stream));
-      fft3d<float2>(S->tmp, S->vol->hv.E, -1, 0, 1, S->vol->tw_f, S->stream, v, none);
-      k_scale<<<cdiv_i(v.N, 256), 256, 0, S->stream>>>(S->tmp, v.N, 1.0f / (float)v.N);
-      CK_LAUNCH();
-      CK(cudaMemcpyAsync(grad, S->tmp, sizeof(float2) * v.N, cudaMemcpyDeviceToHost, S->stream));
-    }
+    if (grad) download_field(S, S->dc.Q + (long long)chain * v.NH, S->dc.Gq, grad);
     CK(cudaStreamSynchronize(S->stream));
   } catch (...) {
     cudaStreamSynchronize(S->stream);
@@ -1900,10 +1948,7 @@ int dr_set_state(dr_chainset* s, int chain, const float* mu, float s_hr, float s
   const int acc = st[chain].acc;
   upload_field(s, mu);
   gather_data(s, s->tmp, chain, acc, true);
-  DevChains none{};
-  fft3d<float2>(s->tmp, s->vol->hv.E, +1, 0, 1, s->vol->tw_f, s->stream, v, none);
-  CK(cudaMemcpyAsync(s->dc.U + ((long long)chain * 2 + acc) * v.N, s->tmp, sizeof(float2) * v.N,
-                     cudaMemcpyDeviceToDevice, s->stream));
+  forward_field(s, s->dc.U + state_off(s, chain, acc), s->dc.G + state_off(s, chain, acc));
   st[chain].sh = s_hr;
   st[chain].ss = s_sr;
   write_states(s, st);
@@ -1911,15 +1956,18 @@ int dr_set_state(dr_chainset* s, int chain, const float* mu, float s_hr, float s
 }
 
 // Checkpoint layout: a header of eight int64 {magic, version, C, N, n_h, n_o, Cp, nsave_stored}, then per chain the
-// accepted spectral state (N float2), mu_D [2][n_h][Cp] and mu_O [2][n_o][Cp] floats, the ChainState array, the
+// accepted spectral state (version 2: the half spectra of Re mu and Im mu, NH float2 each; version 1, still read: the
+// spectrum of mu, N float2), mu_D [2][n_h][Cp] and mu_O [2][n_o][Cp] floats, the ChainState array, the
 // summary sums s1, s2, sa [n_o][Cp] doubles, and with stored samples the samples [nsave][n_o][Cp] floats and the
 // sample records [nsave][C][3] doubles.
 struct CheckpointShape {
   int64_t C, N, n_h, n_o, Cp, nsave;  // nsave: saved-sample capacity when samples are stored, else 0
-  int64_t bytes() const {
+  int64_t NH;
+  int64_t state(int64_t version) const { return version == 1 ? N : 2 * NH; }  // float2 of a chain's spectral state
+  int64_t bytes(int64_t version) const {
     const int64_t no = std::max<int64_t>(n_o, 1);
     int64_t b = 8 * (int64_t)sizeof(int64_t);
-    b += C * N * (int64_t)sizeof(float2);
+    b += C * state(version) * (int64_t)sizeof(float2);
     b += 2 * n_h * Cp * (int64_t)sizeof(float) + 2 * no * Cp * (int64_t)sizeof(float);
     b += C * (int64_t)sizeof(ChainState);
     b += 3 * no * Cp * (int64_t)sizeof(double);
@@ -1927,16 +1975,16 @@ struct CheckpointShape {
     return b;
   }
 };
-static constexpr int64_t CKPT_MAGIC = 0x44524232434b5054LL, CKPT_VERSION = 1;
+static constexpr int64_t CKPT_MAGIC = 0x44524232434b5054LL, CKPT_VERSION = 2;
 
 static CheckpointShape checkpoint_shape(const Chainset* s) {
   const DevVolume& v = s->vol->dv;
   const int64_t nsave = s->opts.store_samples ? std::max(s->opts.nsave, 1) : 0;
-  return CheckpointShape{s->C, v.N, v.n_h, v.n_o, s->dc.Cp, nsave};
+  return CheckpointShape{s->C, v.N, v.n_h, v.n_o, s->dc.Cp, nsave, v.NH};
 }
 
 // Copies between the chain set's device state and the checkpoint buffer (to_host: save; else restore).
-static void checkpoint_copy(Chainset* s, unsigned char* buf, bool to_host) {
+static void checkpoint_copy(Chainset* s, unsigned char* buf, bool to_host, int64_t version = CKPT_VERSION) {
   const CheckpointShape sh = checkpoint_shape(s);
   const DevChains& ch = s->dc;
   const int64_t no = std::max<int64_t>(sh.n_o, 1);
@@ -1952,7 +2000,7 @@ static void checkpoint_copy(Chainset* s, unsigned char* buf, bool to_host) {
   // the chain states first: on restore they say which half of U is each chain's accepted state
   std::vector<ChainState> states(sh.C);
   const size_t u_off = off;
-  off += (size_t)sh.C * sh.N * sizeof(float2);
+  off += (size_t)sh.C * sh.state(version) * sizeof(float2);
   const size_t mu_off = off;
   off += (size_t)(2 * sh.n_h * sh.Cp + 2 * no * sh.Cp) * sizeof(float);
   if (to_host) {
@@ -1964,8 +2012,16 @@ static void checkpoint_copy(Chainset* s, unsigned char* buf, bool to_host) {
   }
   const size_t st_end = off + sizeof(ChainState) * sh.C;
   size_t o = u_off;
-  for (int c = 0; c < sh.C; c++)
-    copy(ch.U + ((int64_t)c * 2 + (states[c].acc & 1)) * sh.N, sizeof(float2) * sh.N, o);
+  for (int c = 0; c < sh.C; c++) {
+    const int64_t at = state_off(s, c, states[c].acc & 1);
+    if (version == 1) {
+      copy(s->tmp, sizeof(float2) * sh.N, o);
+      split_spectrum(s, ch.U + at, ch.G + at);
+    } else {
+      copy(ch.U + at, sizeof(float2) * sh.NH, o);
+      copy(ch.G + at, sizeof(float2) * sh.NH, o);
+    }
+  }
   o = mu_off;
   copy(ch.muD, sizeof(float) * 2 * sh.n_h * sh.Cp, o);
   copy(ch.muO, sizeof(float) * 2 * no * sh.Cp, o);
@@ -1978,12 +2034,12 @@ static void checkpoint_copy(Chainset* s, unsigned char* buf, bool to_host) {
     copy(ch.save_rec, sizeof(double) * sh.nsave * sh.C * 3, o);
   }
   CK(cudaStreamSynchronize(st));
-  if ((int64_t)o != sh.bytes()) throw Error(DR_ERR_STATE, "checkpoint layout mismatch");
+  if ((int64_t)o != sh.bytes(version)) throw Error(DR_ERR_STATE, "checkpoint layout mismatch");
 }
 
 static void checkpoint_save(Chainset* s, void* buf, int64_t bytes) {
   const CheckpointShape sh = checkpoint_shape(s);
-  if (bytes < sh.bytes()) throw Error(DR_ERR_INVALID, "checkpoint buffer too small");
+  if (bytes < sh.bytes(CKPT_VERSION)) throw Error(DR_ERR_INVALID, "checkpoint buffer too small");
   CK(cudaSetDevice(s->vol->device));
   auto* b = static_cast<unsigned char*>(buf);
   const int64_t hdr[8] = {CKPT_MAGIC, CKPT_VERSION, sh.C, sh.N, sh.n_h, sh.n_o, sh.Cp, sh.nsave};
@@ -1996,20 +2052,20 @@ static void checkpoint_restore(Chainset* s, const void* buf, int64_t bytes) {
   if (bytes < 8 * (int64_t)sizeof(int64_t)) throw Error(DR_ERR_INVALID, "checkpoint buffer too small");
   int64_t hdr[8];
   std::memcpy(hdr, buf, sizeof(hdr));
-  if (hdr[0] != CKPT_MAGIC || hdr[1] != CKPT_VERSION) throw Error(DR_ERR_INVALID, "not a chain-set checkpoint");
+  if (hdr[0] != CKPT_MAGIC || hdr[1] < 1 || hdr[1] > CKPT_VERSION) throw Error(DR_ERR_INVALID, "not a chain-set checkpoint");
   const int64_t want[6] = {sh.C, sh.N, sh.n_h, sh.n_o, sh.Cp, sh.nsave};
   for (int i = 0; i < 6; i++)
     if (hdr[2 + i] != want[i])
       throw Error(DR_ERR_INVALID, "checkpoint of a chain set of another shape (chains, volume or stored samples)");
-  if (bytes < sh.bytes()) throw Error(DR_ERR_INVALID, "checkpoint buffer too small");
+  if (bytes < sh.bytes(hdr[1])) throw Error(DR_ERR_INVALID, "checkpoint buffer too small");
   CK(cudaSetDevice(s->vol->device));
-  checkpoint_copy(s, const_cast<unsigned char*>(static_cast<const unsigned char*>(buf)), false);
+  checkpoint_copy(s, const_cast<unsigned char*>(static_cast<const unsigned char*>(buf)), false, hdr[1]);
 }
 
 int dr_chainset_checkpoint_size(const dr_chainset* s, int64_t* bytes) {
   API_BEGIN
   if (!s || !bytes) throw Error(DR_ERR_INVALID, "NULL argument");
-  *bytes = checkpoint_shape(s).bytes();
+  *bytes = checkpoint_shape(s).bytes(CKPT_VERSION);
   API_END
 }
 
@@ -2033,15 +2089,9 @@ int dr_get_state(dr_chainset* s, int chain, float* mu, float* s2inv) {
   CK(cudaSetDevice(s->vol->device));
   std::vector<ChainState> st;
   read_states(s, &st);
-  const DevVolume& v = s->vol->dv;
   if (mu) {
-    CK(cudaMemcpyAsync(s->tmp, s->dc.U + ((long long)chain * 2 + st[chain].acc) * v.N, sizeof(float2) * v.N,
-                       cudaMemcpyDeviceToDevice, s->stream));
-    DevChains none{};
-    fft3d<float2>(s->tmp, s->vol->hv.E, -1, 0, 1, s->vol->tw_f, s->stream, v, none);
-    k_scale<<<cdiv_i(v.N, 256), 256, 0, s->stream>>>(s->tmp, v.N, 1.0f / (float)v.N);
-    CK_LAUNCH();
-    CK(cudaMemcpyAsync(mu, s->tmp, sizeof(float2) * v.N, cudaMemcpyDeviceToHost, s->stream));
+    const long long off = state_off(s, chain, st[chain].acc);
+    download_field(s, s->dc.U + off, s->dc.G + off, mu);
     CK(cudaStreamSynchronize(s->stream));
   }
   if (s2inv) { s2inv[0] = st[chain].sh; s2inv[1] = st[chain].ss; }
@@ -2072,18 +2122,13 @@ int dr_leapfrog_fixed(dr_chainset* s, int chain, const float* mu0, const float* 
   saved = st;
   const DevVolume& v = s->vol->dv;
   const int acc = st[chain].acc;
-  DevChains none{};
   // u0 and the data values of mu0
   upload_field(s, mu0);
   gather_data(s, s->tmp, chain, acc, false);
-  fft3d<float2>(s->tmp, s->vol->hv.E, +1, 0, 1, s->vol->tw_f, s->stream, v, none);
-  CK(cudaMemcpyAsync(s->dc.U + ((long long)chain * 2 + acc) * v.N, s->tmp, sizeof(float2) * v.N,
-                     cudaMemcpyDeviceToDevice, s->stream));
+  forward_field(s, s->dc.U + state_off(s, chain, acc), s->dc.G + state_off(s, chain, acc));
   // q0 = IFFT(p0)
   upload_field(s, p0);
-  fft3d<float2>(s->tmp, s->vol->hv.E, +1, 0, 1, s->vol->tw_f, s->stream, v, none);
-  CK(cudaMemcpyAsync(s->dc.Q + (long long)chain * v.N, s->tmp, sizeof(float2) * v.N, cudaMemcpyDeviceToDevice,
-                     s->stream));
+  forward_field(s, s->dc.Q + (long long)chain * v.NH, s->dc.Gq);
   for (int c = 0; c < s->C; c++) st[c].L_cur = -1;
   st[chain].L_cur = L;
   st[chain].eps_cur = eps;
@@ -2093,11 +2138,12 @@ int dr_leapfrog_fixed(dr_chainset* s, int chain, const float* mu0, const float* 
   const double N = (double)v.N;
   const double sh = st[chain].sh, ss = st[chain].ss;
   if (energies) {
-    const double K0 = part_sum(s, chain, SL_E0, s->dc.nb_x), lp0 = part_sum(s, chain, SL_LP0, s->dc.nb_x);
+    const int ne = s->dc.nb_x + s->dc.nb_g;
+    const double K0 = part_sum(s, chain, SL_E0, ne), lp0 = part_sum(s, chain, SL_LP0, ne);
     const double Rh0 = part_sum(s, chain, SL_RH0, s->dc.nb_wt), RhL = part_sum(s, chain, SL_RHL, s->dc.nb_wt);
     const double Rs0 = v.n_s > 0 ? part_sum(s, chain, SL_RS0, s->dc.nb_w) : 0.0;
     const double RsL = v.n_s > 0 ? part_sum(s, chain, SL_RSL, s->dc.nb_w) : 0.0;
-    const double lpL = part_sum(s, chain, SL_LPL, s->dc.nb_x), KL = part_sum(s, chain, SL_KL, s->dc.nb_x);
+    const double lpL = part_sum(s, chain, SL_LPL, ne), KL = part_sum(s, chain, SL_KL, ne);
     energies[0] = -0.5 * lp0 / N;
     energies[1] = -0.5 * (sh * Rh0 + ss * Rs0);
     energies[2] = -0.5 * K0 / N;
@@ -2106,21 +2152,10 @@ int dr_leapfrog_fixed(dr_chainset* s, int chain, const float* mu0, const float* 
     energies[5] = -0.5 * KL / N;
   }
   if (mu_out) {
-    CK(cudaMemcpyAsync(s->tmp, s->dc.U + ((long long)chain * 2 + (acc ^ 1)) * v.N, sizeof(float2) * v.N,
-                       cudaMemcpyDeviceToDevice, s->stream));
-    fft3d<float2>(s->tmp, s->vol->hv.E, -1, 0, 1, s->vol->tw_f, s->stream, v, none);
-    k_scale<<<cdiv_i(v.N, 256), 256, 0, s->stream>>>(s->tmp, v.N, 1.0f / (float)v.N);
-    CK_LAUNCH();
-    CK(cudaMemcpyAsync(mu_out, s->tmp, sizeof(float2) * v.N, cudaMemcpyDeviceToHost, s->stream));
+    const long long off = state_off(s, chain, acc ^ 1);
+    download_field(s, s->dc.U + off, s->dc.G + off, mu_out);
   }
-  if (p_out) {
-    CK(cudaMemcpyAsync(s->tmp, s->dc.Q + (long long)chain * v.N, sizeof(float2) * v.N, cudaMemcpyDeviceToDevice,
-                       s->stream));
-    fft3d<float2>(s->tmp, s->vol->hv.E, -1, 0, 1, s->vol->tw_f, s->stream, v, none);
-    k_scale<<<cdiv_i(v.N, 256), 256, 0, s->stream>>>(s->tmp, v.N, 1.0f / (float)v.N);
-    CK_LAUNCH();
-    CK(cudaMemcpyAsync(p_out, s->tmp, sizeof(float2) * v.N, cudaMemcpyDeviceToHost, s->stream));
-  }
+  if (p_out) download_field(s, s->dc.Q + (long long)chain * v.NH, s->dc.Gq, p_out);
   CK(cudaStreamSynchronize(s->stream));
   // the chain keeps mu0 as its state; the other chains are untouched
   for (int c = 0; c < s->C; c++) saved[c].L_cur = -1;
@@ -2214,18 +2249,16 @@ int dr_debug_time_kernel(dr_chainset* s, int which, int stp, int reps, double* a
   const DevChains& ch = s->dc;
   const float2* tw = s->vol->tw_f;
   const int C = s->C;
-  const double N = (double)v.N, t1 = (double)ch.t1_stride, t2 = (double)ch.t2_stride, z = (double)s->vol->hv.w_col.size();
+  const double NH = (double)v.NH, t1 = (double)ch.t1_stride, t2 = (double)ch.t2_stride, z = (double)s->vol->hv.w_col.size();
   auto launch = [&]() {
     switch (which) {
       case 0: if (s->plane) launch_plane(s, stp, 0); else launch_xline(s, stp, 0); break;
-      case 1: if (s->plane) break;
-        launch_pass<float2>(v.E1, -1, PRO_LOAD, EPI_STORE, pass_args(ch.T1, ch.T2, ch.t1_stride, ch.t2_stride, v.E2, v.bx, v.E1, v.by, 1.0, stp), v, ch, tw, C, s->stream); break;
-      case 2: launch_pass<float2>(v.E2, -1, PRO_LOAD, EPI_GATHER, pass_args(ch.T2, nullptr, ch.t2_stride, 0, 1, v.by * v.bx, v.E2, v.bz, 1.0 / N, stp, 1, 2), v, ch, tw, C, s->stream); break;
+      case 1: if (!s->plane) launch_y(s, -1, stp); break;
+      case 2: launch_z(-1, zfwd_args(v, stp, 1, 2), v, ch, tw, s->stream); break;
       case 3: if (v.n_s > 0) launch_spmv(s, stp, 1, -1, true); break;
       case 4: launch_spmv(s, stp, 1, -1, false); break;
-      case 5: launch_pass<float2>(v.E2, +1, PRO_DATAGRAD, EPI_STORE, pass_args(nullptr, ch.T2, 0, ch.t2_stride, 1, v.by * v.bx, v.bz, v.E2, 1.0, stp), v, ch, tw, C, s->stream); break;
-      default: if (s->plane) break;
-        launch_pass<float2>(v.E1, +1, PRO_LOAD, EPI_STORE, pass_args(ch.T2, ch.T1, ch.t2_stride, ch.t1_stride, v.E2, v.bx, v.by, v.E1, 1.0, stp), v, ch, tw, C, s->stream); break;
+      case 5: launch_z(+1, zinv_args(stp), v, ch, tw, s->stream); break;
+      default: if (!s->plane) launch_y(s, +1, stp); break;
     }
   };
   launch();  // warm-up
@@ -2247,7 +2280,7 @@ int dr_debug_time_kernel(dr_chainset* s, int which, int stp, int reps, double* a
     const double box = (double)v.bx * v.by * v.bz;
     double b = 0.0;
     switch (which) {
-      case 0: b = C * (2.0 * (s->plane ? t2 : t1) * 8 + 4.0 * N * 8) + N * 4; break;  // T in/out, U and q in/out, 1/lambda
+      case 0: b = C * (2.0 * (s->plane ? t2 : t1) * 8 + 4.0 * NH * 8) + NH * 4; break;  // T in/out, U and q in/out, 1/lambda
       case 1: b = s->plane ? 0.0 : C * (t1 + t2) * 8; break;
       case 2: b = C * (t2 * 8 + (v.n_h + v.n_o) * 4.0) + box * 8; break;            // box maps (2 x int32)
       case 3: b = z * 8 + C * ((double)v.n_h * 4 + (double)v.n_s * 4) + v.n_s * 8.0; // W values + columns, mu_D, rs
@@ -2387,10 +2420,10 @@ static int64_t estimate_bytes(const HostVolume& hv, int C, const dr_hmc_opts& o)
   const double N = (double)hv.N, box = (double)hv.box[0] * hv.box[1] * hv.box[2];
   const double nh = (double)hv.Yh.size(), ns = (double)hv.Ys.size(), no = (double)hv.o_flat.size();
   const double nnz = (double)hv.w_col.size();
-  const double t2 = (double)hv.E[2] * hv.box[1] * hv.box[0];
+  const double ez = hv.E[2] / 2 + 1, NH = ez * hv.E[1] * hv.E[0], t2 = ez * hv.box[1] * hv.box[0];
   double vol = box * 8 + (nh + no) * 4 + (nh + ns) * 4 + (ns + nh + 2) * 4 + nnz * 16 + N * 12 + N * 16;
-  double cs = C * (3 * N * 8 + t2 * 8 + (hv.E[0] == hv.E[1] ? 0.0 : (double)hv.E[2] * hv.E[1] * hv.box[0] * 8)) +
-              C * (2 * (nh + no) * 4 + (nh + ns) * 4 + no * 24) + N * 8 + (double)C * 9 * 2048 * 8;
+  double cs = C * (5 * NH * 8 + t2 * 8 + (hv.E[0] == hv.E[1] ? 0.0 : ez * hv.E[1] * hv.box[0] * 8)) +
+              C * (2 * (nh + no) * 4 + (nh + ns) * 4 + no * 24) + N * 8 + NH * 8 + (double)C * 9 * 2048 * 8;
   if (o.store_samples) cs += (double)std::max(o.nsave, 1) * (no * 4 + 24) * C;
   if (tc_chains(C) > 0 && ns > 0) {
     // dense tiles of W and W^T for the tensor-core products (their column unions are a few times the nonzeros:
@@ -2534,7 +2567,7 @@ struct Server {
   // set-up for the rebuild, and marks it preempted.
   void preempt(const std::shared_ptr<Job>& j) {
     Chainset* cs = j->cs.get();
-    const int64_t n = checkpoint_shape(cs).bytes();
+    const int64_t n = checkpoint_shape(cs).bytes(CKPT_VERSION);
     std::vector<unsigned char> buf((size_t)n);
     checkpoint_save(cs, buf.data(), n);
     HostVolume hv = std::move(j->vol->hv);
@@ -3117,8 +3150,7 @@ extern "C" int dr_log_posterior_noalloc(const dr_volume* v, const float* mu_devi
   launch_spmv_dc(dv, ch, 1, -1, 0, 0, false, s);
   // u = IFFT(mu) in the scratch field, then the prior's spectral sum
   CK(cudaMemcpyAsync(field, mu_device, sizeof(float2) * dv.N, cudaMemcpyDeviceToDevice, s));
-  DevChains none{};
-  fft3d<float2>(field, v->hv.E, +1, 0, 1, v->tw_f, s, dv, none);
+  fft3d<float2>(field, v->hv.E, +1, v->tw_f, s);
   double* epart = (double*)(base + NA_EPART);
   k_spectral_energy<<<NA_EBLK, 256, 0, s>>>(field, dv.sinv, dv.N, s_hr, 0, epart);
   CK_LAUNCH();

@@ -52,6 +52,8 @@ struct ChainState {
 struct DevVolume {
   int E0, E1, E2;
   long long N;
+  int EZ;                   // spectral planes kept: 0 .. E2/2
+  long long NH;             // modes of the half spectrum, EZ * E1 * E0
   int bx, by, bz;           // real-space box covering data and output voxels
   int n_h, n_s, n_o;
   const float* sinv;        // [N] 1/Re(lambda) on live modes, -1 on S
@@ -74,10 +76,12 @@ struct DevChains {
   int C;                    // chains
   int Cp;                   // pitch of the chain-minor arrays (>= C)
   int CG;                   // lanes per chain group in the kriging kernels (power of two <= 32)
-  float2* U;                // [C][2][N]  spectral state: accepted / proposal halves
-  float2* Q;                // [C][N]     spectral momentum
-  float2* T1;               // [C][E2*E1*bx]
-  float2* T2;               // [C][E2*by*bx]
+  float2* U;                // [C][2][NH] half spectrum of Re mu: accepted / proposal halves
+  float2* G;                // [C][2][NH] half spectrum of Im mu, the same
+  float2* Q;                // [C][NH]    half-spectrum momentum of Re mu (that of Im mu lives in k_momentum's registers)
+  float2* Gq;               // [NH]       given momentum of Im mu (fixed-momentum calls, one chain)
+  float2* T1;               // [C][EZ*E1*bx]
+  float2* T2;               // [C][EZ*by*bx]
   long long t1_stride, t2_stride;
   float* muD;               // [2][n_h][Cp] Re mu at data voxels
   float* muO;               // [2][n_o][Cp] Re mu at output voxels
@@ -85,7 +89,8 @@ struct DevChains {
   float* rs;                // [n_s][Cp] Ys - W mu_D
   double* part;             // [C][NSLOT][maxblk]
   int maxblk;
-  int nb_x, nb_w, nb_wt;    // blocks writing partials in the x-line / W / W^T kernels
+  int nb_x, nb_w, nb_wt;    // blocks writing partials in the update / W / W^T kernels
+  int nb_g;                 // blocks of k_momentum: their partials follow the update kernel's
   ChainState* st;           // [C]
   double* s1;               // [n_o][Cp] sum mu
   double* s2;               // [n_o][Cp] sum mu^2
@@ -127,15 +132,16 @@ struct PassArgs {
   void* out;
   long long in_cs, out_cs;  // per-chain strides (complex elements)
   int A, B, n_in, n_out;
-  double scale;
   int step;                 // hot-path step for chain masking; -1 = all chains
-  int sel;                  // 0: accepted half of muD/muO; 1: proposal half
-  int write_o;              // gather epilogue: 0 never, 1 always, 2 when step == L_cur
-  int chain_only;           // >= 0: only this chain (API calls); -1: all
 };
 
-enum PassPro : int { PRO_LOAD = 0, PRO_DATAGRAD = 1 };
-enum PassEpi : int { EPI_STORE = 0, EPI_GATHER = 1 };
+// z-pass arguments (k_zinv, k_zfwd).
+struct ZArgs {
+  int step;                 // hot-path step for chain masking; -1 = all chains
+  int sel;                  // 0: accepted half of muD/muO; 1: proposal half
+  int write_o;              // k_zfwd: mu_O 0 never, 1 always, 2 when step == L_cur
+  float scale;              // k_zfwd: factor of the transformed values
+};
 
 // x-line kernel flags
 // XF_L2_PREFETCH: the update kernels ask L2 for their blocks' state (u, q, 1/lambda) at entry, so that its DRAM

@@ -12,6 +12,18 @@
 // scatter of the data gradient.  One gradient therefore costs one pruned
 // forward transform (spectral -> real box) and one pruned inverse transform
 // (real box -> spectral) instead of the reference's four full 3D FFTs.
+//
+// The state is split into the spectra of Re mu and Im mu, u = h + i g, each
+// Hermitian (h(-k) = conj h(k)), so the planes kz = 0 .. E2/2 hold all of it:
+// EZ = E2/2 + 1 planes, NH = EZ E1 E0 modes.  lambda is even in every axis, so
+// the operators above act on h and g alike and never mix them.  Only h meets
+// the data: the leapfrog steps carry h (half the modes through every kernel),
+// and g, whose dynamics are element-wise and linear, is taken through all of an
+// iteration's steps in registers by k_momentum.  Sums over all modes weight the
+// planes 0 < kz < E2/2 by two (plane_weight).  Measured against the full complex
+// state (64 chains on a 64^3 embedding): update 139 -> 73 us, forward / inverse z
+// pass 20.4 / 18.1 -> 10.6 / 10.1 us, an iteration 6.1 -> 4.1 ms; 16 chains on
+// 128^3: update 458 -> 252 us, z 38 / 34 -> 16 / 17 us.
 #include "common.cuh"
 #include "drb.h"
 #include "fft.cuh"
@@ -22,6 +34,9 @@ namespace drb {
 // e / d as __umulhi(e, box_div_magic(d)) for box positions (e < 2^15, 2 <= d <= 1024): the multiplier
 // ceil(2^32 / d) gives the exact quotient there, without a division per element.
 __device__ __forceinline__ uint32_t box_div_magic(int d) { return 0xFFFFFFFFu / (uint32_t)d + 1u; }
+
+// Multiplicity of spectral plane z in a sum over all modes: its mirror image E2 - z is not stored.
+__device__ __forceinline__ double plane_weight(int z, int E2) { return (z == 0 || 2 * z == E2) ? 1.0 : 2.0; }
 
 // ----------------------------------------------------------------- twiddles
 __device__ float2 g_tw_f[TW_TOTAL];
@@ -99,77 +114,44 @@ __device__ double gamma_draw(double shape, double scale, uint64_t seed, uint32_t
 
 // ----------------------------------------------------------------- pass kernel
 // Batched 1D FFT along the middle axis of [A][n][B] arrays, one tile of 32
-// lines (line = a * B + b) per block.  CPB = 1: the 32 lines of one chain
-// (blockIdx.y).  CPB = 8: 4 consecutive lines of 8 chains (chain group
-// blockIdx.y), used by the z passes whose epilogue / prologue touch the
-// chain-minor arrays mu_D, mu_O and gD: a warp then reads and writes 8 chains
-// x 4 bytes contiguously there, instead of one 4-byte value per 256-byte row,
-// while its T2 accesses stay whole 32-byte sectors (4 lines x 8 bytes).
+// lines (line = a * B + b) of one chain (blockIdx.y) per block: the y passes of
+// the x-line path, the initial state and the unpruned 3D transforms.
 template <int N> struct PassCfg {
   static constexpr int NT = N >= 512 ? 512 : 256;
 };
 
-template <int N, int DIR, int PRO, int EPI, class C, int CPB = 1, int PLAN = 0>
-__global__ void __launch_bounds__(PassCfg<N>::NT) k_pass(PassArgs a, DevVolume v, DevChains ch, const C* __restrict__ tw) {
+template <int N, int DIR, class C>
+__global__ void __launch_bounds__(PassCfg<N>::NT) k_pass(PassArgs a, DevChains ch, const C* __restrict__ tw) {
   grid_dep_wait();
-  constexpr int TL = TILE_LINES, P = TILE_LINES + 1, NT = PassCfg<N>::NT, LPC = TILE_LINES / CPB;
+  constexpr int TL = TILE_LINES, P = TILE_LINES + 1, NT = PassCfg<N>::NT;
   extern __shared__ __align__(16) unsigned char smraw[];
   C* sm = reinterpret_cast<C*>(smraw);
-  __shared__ int s_ok[CPB], s_hsel[CPB], s_wo[CPB];
   __shared__ long long s_in0[TL], s_out0[TL];  // per tile line: index of its element 0 in the input / output
-  const int cbase = CPB == 1 ? ((a.chain_only >= 0) ? a.chain_only : (int)blockIdx.y) : (int)blockIdx.y * CPB;
-  if (threadIdx.x < CPB) {
-    // per chain of the tile: active at this step, the half of mu_D / mu_O written, whether mu_O is written
-    const int c = cbase + (int)threadIdx.x;
-    int ok = CPB == 1 || c < ch.C;
-    if (ok && a.step >= 0 && ch.st != nullptr && a.step > ch.st[c].L_cur) ok = 0;
-    s_ok[threadIdx.x] = ok;
-    int hs = 0, wo = 0;
-    if (EPI == EPI_GATHER && ok) {
-      hs = (ch.st != nullptr ? ch.st[c].acc : 0) ^ a.sel;
-      wo = a.write_o == 1 || (a.write_o == 2 && ch.st != nullptr && a.step == ch.st[c].L_cur);
-    }
-    s_hsel[threadIdx.x] = hs;
-    s_wo[threadIdx.x] = wo;
-  }
+  const int c = blockIdx.y;
+  if (a.step >= 0 && ch.st != nullptr && a.step > ch.st[c].L_cur) return;
   const long long lines = (long long)a.A * a.B;
-  const long long l0 = (long long)blockIdx.x * LPC;
+  const long long l0 = (long long)blockIdx.x * TL;
   const int B = a.B, n_in = a.n_in, n_out = a.n_out;
   if (threadIdx.x < TL) {
     // line lam = a * B + b starts at (a * n) * B + b; computed once per line rather than per element
-    const long long lam = l0 + threadIdx.x % LPC;
+    const long long lam = l0 + threadIdx.x;
     const long long aa = lam / B, bb = lam - aa * B;
     s_in0[threadIdx.x] = aa * n_in * B + bb;
     s_out0[threadIdx.x] = aa * n_out * B + bb;
   }
   __syncthreads();
-  if (CPB == 1 && !s_ok[0]) return;
-  const int nl = (int)min((long long)LPC, lines - l0);
-  // tile line l: chain slot l / LPC of the tile, line l0 + l % LPC
-  auto valid = [&](int l) { return (l % LPC) < nl && s_ok[l / LPC]; };
-  auto chain = [&](int l) { return cbase + l / LPC; };
-  auto in_index = [&](int l, int i) -> long long { return s_in0[l] + (long long)i * B; };
-  auto out_index = [&](int l, int k) -> long long { return s_out0[l] + (long long)k * B; };
-  // bounds of the data-dependent indices (checked builds only): a chain's stride in the input / output (the whole
-  // array when there is one field), the box, the data and output voxels
+  const int nl = (int)min((long long)TL, lines - l0);
+  // bounds of the indices (checked builds only): a chain's stride in the input / output (the whole array when there is
+  // one field)
   const long long in_lim = a.in_cs > 0 ? a.in_cs : 0x7fffffffffffffffLL;
   const long long out_lim = a.out_cs > 0 ? a.out_cs : 0x7fffffffffffffffLL;
-  const long long box = (long long)v.bx * v.by * v.bz;
+  const C* in = reinterpret_cast<const C*>(a.in) + (long long)c * a.in_cs;
+  C* out = reinterpret_cast<C*>(a.out) + (long long)c * a.out_cs;
   auto load = [&](int l, int i) -> C {
     C val = mk((decltype(C().x))0, (decltype(C().x))0);
-    if (valid(l) && i < n_in) {
-      const long long idx = in_index(l, i);
-      const int c = chain(l);
-      if (PRO == PRO_LOAD) {
-        // the forward z pass is the last reader of its input (T2): streaming loads, evicted first
-        if (in_bounds(idx, in_lim, ch.err)) {
-          if constexpr (EPI == EPI_GATHER) val = __ldcs(reinterpret_cast<const C*>(a.in) + (long long)c * a.in_cs + idx);
-          else val = reinterpret_cast<const C*>(a.in)[(long long)c * a.in_cs + idx];
-        }
-      } else if (in_bounds(idx, box, ch.err)) {
-        const int j = v.box_to_d[idx];
-        if (j >= 0 && in_bounds(j, v.n_h, ch.err)) val.x = ch.gD[(long long)j * ch.Cp + c];
-      }
+    if (l < nl && i < n_in) {
+      const long long idx = s_in0[l] + (long long)i * B;
+      if (in_bounds(idx, in_lim, ch.err)) val = in[idx];
     }
     return val;
   };
@@ -205,28 +187,12 @@ __global__ void __launch_bounds__(PassCfg<N>::NT) k_pass(PassArgs a, DevVolume v
     }
   }
   __syncthreads();
-  fft_smem<N, DIR, TL, NT, C, PLAN>(sm, 1, P, TL, tw + tw_offset(N));
+  fft_smem<N, DIR, TL, NT, C>(sm, 1, P, TL, tw + tw_offset(N));
 
-  const auto scale = (decltype(C().x))a.scale;
   auto store = [&](int l, int k) {
-    if (!valid(l) || k >= n_out) return;
-    const long long idx = out_index(l, k);
-    const int c = chain(l);
-    const C val = sm[k * P + l];
-    if (EPI == EPI_STORE) {
-      if (in_bounds(idx, out_lim, ch.err))
-        reinterpret_cast<C*>(a.out)[(long long)c * a.out_cs + idx] = mk(val.x * scale, val.y * scale);
-    } else if (in_bounds(idx, box, ch.err)) {
-      const int slot = l / LPC;
-      const int j = v.box_to_d[idx];
-      if (j >= 0 && in_bounds(j, v.n_h, ch.err))
-        ch.muD[((long long)s_hsel[slot] * v.n_h + j) * ch.Cp + c] = (float)(val.x * scale);
-      if (s_wo[slot]) {
-        const int o = v.box_to_o[idx];
-        if (o >= 0 && in_bounds(o, v.n_o, ch.err))
-          ch.muO[((long long)s_hsel[slot] * v.n_o + o) * ch.Cp + c] = (float)(val.x * scale);
-      }
-    }
+    if (l >= nl || k >= n_out) return;
+    const long long idx = s_out0[l] + (long long)k * B;
+    if (in_bounds(idx, out_lim, ch.err)) out[idx] = sm[k * P + l];
   };
   if (B == 1) {
     for (int e = threadIdx.x; e < TL * N; e += NT) store(e / N, e % N);
@@ -235,13 +201,299 @@ __global__ void __launch_bounds__(PassCfg<N>::NT) k_pass(PassArgs a, DevVolume v
   }
 }
 
+// ----------------------------------------------------------------- z passes
+// The z transforms between the real box and T2 (the planes 0 .. E2/2 of its
+// half spectrum along z).  A tile line is a pair of x-adjacent real lines a, b
+// carried as one complex line a + i b, so one transform of length E2 serves two
+// lines and T2 moves as float4 (the pair's A(k), B(k)):
+//   inverse  gD in the box -> Z, then A(k) = (Z(k) + conj Z(-k)) / 2 and
+//            B(k) = (Z(k) - conj Z(-k)) / 2i for k = 0 .. E2/2;
+//   forward  Z(k) = A(k) + i B(k), Z(-k) = conj A(k) + i conj B(k), whose
+//            transform's real and imaginary parts are Re mu on the two lines
+//            (in the planes k = 0 and E2/2, real for a real field, the real parts are taken).
+// CPB = 1: TL pair lines of one chain (blockIdx.y): 32, or 8 when 32 would give
+// fewer blocks than two per SM.  CPB = 8: 4 consecutive pair lines of 8 chains
+// (chain group blockIdx.y): the chain-minor arrays mu_D, mu_O and gD are then
+// touched 8 chains x 4 bytes contiguously, one 32-byte sector instead of one
+// value per 256-byte row, and T2 in runs of 64 bytes.
+template <int N, int TL> struct ZCfg {
+  static constexpr int WANT = TL * N / 8;  // a thread holds 8 elements
+  static constexpr int NT = WANT < 32 ? 32 : (WANT > 256 ? 256 : WANT);
+  static constexpr int P = TL;             // element pitch: threads run along the lines, whole rows at a time
+  static constexpr int SMEM = N * P * 8;
+};
+
+// Per chain of a tile: whether it takes part in this step.
+template <int CPB>
+__device__ __forceinline__ bool z_chain_active(const ZArgs& a, const DevChains& ch, int c) {
+  if (CPB > 1 && c >= ch.C) return false;
+  return a.step < 0 || ch.st == nullptr || a.step <= ch.st[c].L_cur;
+}
+
+template <int N, int TL, int CPB, int PLAN>
+__global__ void __launch_bounds__(ZCfg<N, TL>::NT) k_zinv(ZArgs a, DevVolume v, DevChains ch, const float2* __restrict__ tw) {
+  grid_dep_wait();
+  constexpr int NT = ZCfg<N, TL>::NT, P = ZCfg<N, TL>::P, LPC = TL / CPB, H = N / 2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float2* sm = reinterpret_cast<float2*>(smraw);
+  const int l = threadIdx.x % TL;          // NT is a multiple of TL: a thread keeps its line
+  constexpr int KS = NT / TL;              // elements between a thread's consecutive ones
+  const int c = blockIdx.y * CPB + l / LPC;
+  const int lp = blockIdx.x * LPC + l % LPC;
+  const bool act = z_chain_active<CPB>(a, ch, c);
+  if (CPB == 1 && !act) return;
+  const int plane = v.by * v.bx;
+  const bool on = act && 2 * lp < plane;
+  const long long box = (long long)plane * v.bz;
+  constexpr int PER = (N + KS - 1) / KS, CH = PER > 8 ? 8 : PER;
+  const int k0 = threadIdx.x / TL;
+#pragma unroll 1
+  for (int q0 = 0; q0 < PER; q0 += CH) {
+    int2 j[CH];
+#pragma unroll
+    for (int q = 0; q < CH; q++) {
+      const int z = k0 + (q0 + q) * KS;
+      const long long idx = (long long)z * plane + 2 * lp;
+      j[q] = make_int2(-1, -1);
+      if (on && z < v.bz && in_bounds(idx + 1, box, ch.err)) j[q] = __ldg(reinterpret_cast<const int2*>(v.box_to_d + idx));
+    }
+    float2 r[CH];
+#pragma unroll
+    for (int q = 0; q < CH; q++) {
+      r[q] = make_float2(0.f, 0.f);
+      if (j[q].x >= 0 && in_bounds(j[q].x, v.n_h, ch.err)) r[q].x = ch.gD[(long long)j[q].x * ch.Cp + c];
+      if (j[q].y >= 0 && in_bounds(j[q].y, v.n_h, ch.err)) r[q].y = ch.gD[(long long)j[q].y * ch.Cp + c];
+    }
+#pragma unroll
+    for (int q = 0; q < CH; q++)
+      if (N % KS == 0 || k0 + (q0 + q) * KS < N) sm[(k0 + (q0 + q) * KS) * P + l] = r[q];
+  }
+  __syncthreads();
+  fft_smem<N, +1, TL, NT, float2, PLAN>(sm, 1, P, TL, tw + tw_offset(N));
+  if (!on) return;
+  float2* T = ch.T2 + (long long)c * ch.t2_stride + 2 * lp;
+  for (int k = k0; k <= H; k += KS) {
+    const float2 zk = sm[k * P + l], zm = sm[((N - k) % N) * P + l];
+    if (in_bounds((long long)k * plane + 2 * lp + 1, ch.t2_stride, ch.err))
+      *reinterpret_cast<float4*>(T + (long long)k * plane) =
+          make_float4(0.5f * (zk.x + zm.x), 0.5f * (zk.y - zm.y), 0.5f * (zk.y + zm.y), 0.5f * (zm.x - zk.x));
+  }
+}
+
+template <int N, int TL, int CPB, int PLAN>
+__global__ void __launch_bounds__(ZCfg<N, TL>::NT) k_zfwd(ZArgs a, DevVolume v, DevChains ch, const float2* __restrict__ tw) {
+  grid_dep_wait();
+  constexpr int NT = ZCfg<N, TL>::NT, P = ZCfg<N, TL>::P, LPC = TL / CPB, H = N / 2;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  float2* sm = reinterpret_cast<float2*>(smraw);
+  const int l = threadIdx.x % TL;
+  constexpr int KS = NT / TL;
+  const int c = blockIdx.y * CPB + l / LPC;
+  const int lp = blockIdx.x * LPC + l % LPC;
+  const bool act = z_chain_active<CPB>(a, ch, c);
+  if (CPB == 1 && !act) return;
+  const int plane = v.by * v.bx;
+  const bool on = act && 2 * lp < plane;
+  const float2* T = ch.T2 + (long long)c * ch.t2_stride + 2 * lp;
+  const int k0 = threadIdx.x / TL;
+  // T2 is read for the last time before the next inverse z pass: streaming loads, evicted first
+  auto load = [&](int k) {
+    if (on && k <= H && in_bounds((long long)k * plane + 2 * lp + 1, ch.t2_stride, ch.err))
+      return __ldcs(reinterpret_cast<const float4*>(T + (long long)k * plane));
+    return make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  // k = 0 .. H-1 over the threads, and the threads of k = 0 also take k = H
+  constexpr int PER = (H + KS - 1) / KS, CH = PER > 4 ? 4 : PER;
+  float4 rh = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (k0 == 0) rh = load(H);
+#pragma unroll 1
+  for (int q0 = 0; q0 < PER; q0 += CH) {
+    float4 r[CH];
+#pragma unroll
+    for (int q = 0; q < CH; q++) r[q] = load(k0 + (q0 + q) * KS);
+#pragma unroll
+    for (int q = 0; q < CH; q++) {
+      const int k = k0 + (q0 + q) * KS;
+      if (k == 0) {
+        sm[l] = make_float2(r[q].x, r[q].z);
+      } else if (k < H) {
+        sm[k * P + l] = make_float2(r[q].x - r[q].w, r[q].y + r[q].z);
+        sm[(N - k) * P + l] = make_float2(r[q].x + r[q].w, r[q].z - r[q].y);
+      }
+    }
+  }
+  if (k0 == 0) sm[H * P + l] = make_float2(rh.x, rh.z);
+  __syncthreads();
+  fft_smem<N, -1, TL, NT, float2, PLAN>(sm, 1, P, TL, tw + tw_offset(N));
+  if (!on) return;
+  // the half of mu_D / mu_O that is written, and whether mu_O is
+  int half = a.sel, wo = a.write_o == 1;
+  if (ch.st != nullptr) {
+    half ^= ch.st[c].acc;
+    wo |= a.write_o == 2 && a.step == ch.st[c].L_cur;
+  }
+  float* mD = ch.muD + (long long)half * v.n_h * ch.Cp + c;
+  float* mO = ch.muO + (long long)half * v.n_o * ch.Cp + c;
+  const long long box = (long long)plane * v.bz;
+  for (int z = k0; z < v.bz; z += KS) {
+    const long long idx = (long long)z * plane + 2 * lp;
+    if (!in_bounds(idx + 1, box, ch.err)) continue;
+    const float2 m = cscale(sm[z * P + l], a.scale);
+    const int2 j = __ldg(reinterpret_cast<const int2*>(v.box_to_d + idx));
+    if (j.x >= 0 && in_bounds(j.x, v.n_h, ch.err)) mD[(long long)j.x * ch.Cp] = m.x;
+    if (j.y >= 0 && in_bounds(j.y, v.n_h, ch.err)) mD[(long long)j.y * ch.Cp] = m.y;
+    if (wo) {
+      const int2 o = __ldg(reinterpret_cast<const int2*>(v.box_to_o + idx));
+      if (o.x >= 0 && in_bounds(o.x, v.n_o, ch.err)) mO[(long long)o.x * ch.Cp] = m.x;
+      if (o.y >= 0 && in_bounds(o.y, v.n_o, ch.err)) mO[(long long)o.y * ch.Cp] = m.y;
+    }
+  }
+}
+
+// ----------------------------------------------------------------- momentum and Im mu
+// One launch per iteration, before its leapfrog steps, over the rows (z, y) of
+// the half spectrum.  It draws the momentum (MultiResParameters.h:784-815),
+// q = sqrt(N lambda_m) w with w(k) ~ CN(0, 2) iid over all N modes, as in the
+// full spectrum (one Philox call per pair of x-adjacent modes), and splits it:
+//   h part  sqrt(N lambda_m) (w(k) + conj w(-k)) / 2  -> Q, for the leapfrog kernels;
+//   g part  sqrt(N lambda_m) (w(k) - conj w(-k)) / 2i, kept here.
+// The g part of the state (Im mu) feels only the prior, so its whole trajectory
+//   q -= (eps / 2) u / lambda;  L times { u += eps q / lambda_m;  q -= eps u / lambda (the last one halved) }
+// is element-wise: it runs here in registers, 4 FMA per component and step, and
+// reads and writes g once per iteration instead of once per step.  Energies of
+// the g part and sum |w|^2 go to partial-sum entries nb_x + block (the leapfrog
+// kernels' entries are 0 .. nb_x - 1).
+// FIXED: the g part of a given momentum is read from Gq and left there (the h
+// part is in Q), and SL_E0 receives sum |q|^2 / lambda_m; one chain at a time.
+constexpr int MOM_ITEMS = 512;  // modes of a row group: 512 / E0 rows
+constexpr int MOM_NT = 256;
+
+template <bool FIXED>
+__global__ void __launch_bounds__(MOM_NT) k_momentum(DevVolume v, DevChains ch) {
+  grid_dep_wait();
+  __shared__ float2 wa[FIXED ? 1 : MOM_ITEMS], wb[FIXED ? 1 : MOM_ITEMS];
+  __shared__ double red[MOM_NT / 32];
+  const int c = blockIdx.y;
+  const ChainState& st = ch.st[c];
+  const int L = st.L_cur;
+  if (L < 0) return;
+  const int E0 = v.E0, E1 = v.E1, E2 = v.E2, acc = st.acc;
+  const long long NH = v.NH;
+  const float eps = st.eps_cur, sh = st.sh, Nf = (float)v.N;
+  const float2* Gs = ch.G + ((long long)c * 2 + acc) * NH;
+  float2* Gd = ch.G + ((long long)c * 2 + (acc ^ 1)) * NH;
+  float2* Qc = ch.Q + (long long)c * NH;
+  double e0 = 0.0, lp0 = 0.0, lpl = 0.0, kl = 0.0;
+  const int rows = v.EZ * E1, rpg = MOM_ITEMS / E0;  // E0 is a power of two <= 256
+  for (int r0 = blockIdx.x * rpg; r0 < rows; r0 += gridDim.x * rpg) {
+    const int nr = min(rpg, rows - r0), items = nr * E0;
+    if constexpr (!FIXED) {
+      __syncthreads();
+      for (int p = threadIdx.x; p < items; p += MOM_NT) {
+        // pairs of modes: the rows themselves, then their mirror images
+        const int which = 2 * p >= items, i = 2 * p - which * items, row = r0 + i / E0, x = i % E0;
+        int z = row / E1, y = row % E1;
+        if (which) {
+          z = z == 0 ? 0 : E2 - z;
+          y = y == 0 ? 0 : E1 - y;
+        }
+        const long long gi = ((long long)z * E1 + y) * E0 + x;
+        const u32x4 r = philox(u32x4{(uint32_t)(gi >> 1), (uint32_t)st.iteration, (uint32_t)(ch.chain0 + c),
+                                     RNG_MOMENTUM}, ch.seed);
+        float2* w = which ? wb : wa;
+        w[i] = box_muller(u01f(r.x), u01f(r.y));
+        w[i + 1] = box_muller(u01f(r.z), u01f(r.w));
+      }
+      __syncthreads();
+    }
+    for (int i = threadIdx.x; i < items; i += MOM_NT) {
+      const int row = r0 + i / E0;
+      const long long gi = (long long)r0 * E0 + i;
+      const double wt = plane_weight(row / E1, E2);
+      float2 u = __ldcs(Gs + gi);
+      const float s = v.sinv[gi];
+      const bool live = s > 0.0f;
+      const float lm = s + sh;  // lambda_m = 1/lambda + sigma_h^-2 (MultiResParameters.h:735-738)
+      float2 q;
+      if constexpr (FIXED) {
+        q = ch.Gq[gi];
+        if (live) e0 += wt * ((double)(q.x * q.x + q.y * q.y) / (double)lm);
+      } else {
+        const int x = i % E0;
+        const float2 w = wa[i], m = wb[i - x + (x == 0 ? 0 : E0 - x)];
+        const float a = live ? 0.5f * sqrtf(Nf * lm) : 0.0f;
+        // sum |w|^2 over all modes: each mode of the mirror plane is some m of this plane
+        e0 += (double)(w.x * w.x + w.y * w.y);
+        if (wt > 1.0) e0 += (double)(m.x * m.x + m.y * m.y);
+        Qc[gi] = make_float2(a * (w.x + m.x), a * (w.y - m.y));
+        q = make_float2(a * (w.y + m.y), a * (m.x - w.x));
+      }
+      if (live) {
+        lp0 += wt * ((double)(u.x * u.x + u.y * u.y) * (double)s);
+        const float kick = eps * s, half = 0.5f * kick, drift = eps / lm;
+        q.x = fmaf(-half, u.x, q.x);
+        q.y = fmaf(-half, u.y, q.y);
+#pragma unroll 4
+        for (int t = 1; t < L; t++) {
+          u.x = fmaf(drift, q.x, u.x);
+          u.y = fmaf(drift, q.y, u.y);
+          q.x = fmaf(-kick, u.x, q.x);
+          q.y = fmaf(-kick, u.y, q.y);
+        }
+        if (L > 0) {
+          u.x = fmaf(drift, q.x, u.x);
+          u.y = fmaf(drift, q.y, u.y);
+          q.x = fmaf(-half, u.x, q.x);
+          q.y = fmaf(-half, u.y, q.y);
+        }
+        lpl += wt * ((double)(u.x * u.x + u.y * u.y) * (double)s);
+        kl += wt * ((double)(q.x * q.x + q.y * q.y) / (double)lm);
+      }
+      if (L > 0) __stcs(Gd + gi, u);  // an evaluation (L = 0) leaves the state as it is
+      if constexpr (FIXED) ch.Gq[gi] = q;
+    }
+  }
+  const double sums[4] = {e0, lp0, lpl, kl};
+  const int slots[4] = {SL_E0, SL_LP0, SL_LPL, SL_KL};
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const double t = block_sum(sums[k], red);
+    if (threadIdx.x == 0) ch.part[((long long)c * NSLOT + slots[k]) * ch.maxblk + ch.nb_x + blockIdx.x] = t;
+  }
+}
+
+// u = h + i g on all N modes <-> the half spectra.  A mode k of a plane z > E2/2 is conj of -k.
+__global__ void k_merge(DevVolume v, const float2* __restrict__ h, const float2* __restrict__ g, float2* __restrict__ u) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= v.N) return;
+  const int x = (int)(i % v.E0), y = (int)((i / v.E0) % v.E1), z = (int)(i / ((long long)v.E0 * v.E1));
+  long long j = i;
+  float sg = 1.0f;
+  if (z >= v.EZ) {
+    j = ((long long)(v.E2 - z) * v.E1 + (y == 0 ? 0 : v.E1 - y)) * v.E0 + (x == 0 ? 0 : v.E0 - x);
+    sg = -1.0f;
+  }
+  const float2 a = h[j], b = g[j];
+  u[i] = make_float2(a.x - sg * b.y, sg * a.y + b.x);
+}
+__global__ void k_split(DevVolume v, const float2* __restrict__ u, float2* __restrict__ h, float2* __restrict__ g) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= v.NH) return;
+  const int x = (int)(i % v.E0), y = (int)((i / v.E0) % v.E1), z = (int)(i / ((long long)v.E0 * v.E1));
+  const long long j = ((long long)(z == 0 ? 0 : v.E2 - z) * v.E1 + (y == 0 ? 0 : v.E1 - y)) * v.E0 + (x == 0 ? 0 : v.E0 - x);
+  const float2 a = u[i], m = u[j];
+  h[i] = make_float2(0.5f * (a.x + m.x), 0.5f * (a.y - m.y));
+  g[i] = make_float2(0.5f * (a.y + m.y), 0.5f * (m.x - a.x));
+}
+
 // ----------------------------------------------------------------- x-line kernel
 // The hot kernel of one leapfrog step, for 32 x-lines of one chain:
 //   inverse x-FFT of the data gradient (spectral except along x),
 //   kick  q += k eps (IFFT(data grad) - u / lambda)          (MultiResParameters.h:690, 699)
 //   drift u* += eps q / lambda_m                              (:693-698)
 //   forward x-FFT of u* for the next gradient.
-// Step 0 also draws the momentum (:784-815) and the initial energies; the
+// Step 0 starts from the momentum that k_momentum drew and adds the initial
+// energies; the
 // last step only kicks and accumulates the final energies (:702-705).
 template <int E0> struct XCfg {
   static constexpr int NT = E0 >= 512 ? 512 : 256;
@@ -265,24 +517,23 @@ __global__ void __launch_bounds__(XCfg<E0>::NT, XCfg<E0>::MINB) k_xline(DevVolum
   const bool first = step == 0, last = step == Lc;
   const float eps = st.eps_cur, sh = st.sh;
   const int acc = st.acc;
-  const long long N = v.N;
-  const long long lines = (long long)v.E1 * v.E2;
+  const long long NH = v.NH;
+  const long long lines = (long long)v.E1 * v.EZ;
   const long long lam0 = (long long)blockIdx.x * TL;
   // the block's lines of the state and of T1 lie in their arrays (checked builds)
-  if (!in_bounds(min(lam0 + TL, lines) * E0 - 1, N, ch.err) ||
+  if (!in_bounds(min(lam0 + TL, lines) * E0 - 1, NH, ch.err) ||
       !in_bounds(min(lam0 + TL, lines) * v.bx - 1, ch.t1_stride, ch.err))
     return;
   const int nl = (int)min((long long)TL, lines - lam0);
-  float2* Ub = ch.U + (long long)c * 2 * N;
-  const float2* Usrc = Ub + (long long)(first ? acc : (acc ^ 1)) * N;
-  float2* Udst = Ub + (long long)(acc ^ 1) * N;
-  float2* Qc = ch.Q + (long long)c * N;
+  float2* Ub = ch.U + (long long)c * 2 * NH;
+  const float2* Usrc = Ub + (long long)(first ? acc : (acc ^ 1)) * NH;
+  float2* Udst = Ub + (long long)(acc ^ 1) * NH;
+  float2* Qc = ch.Q + (long long)c * NH;
   float2* T1 = ch.T1 + (long long)c * ch.t1_stride;
   const int bx = v.bx;
   if ((flags & XF_L2_PREFETCH) && threadIdx.x == 0 && E0 >= 4) {
-    const bool draw = first && !(flags & XF_FIXED_MOMENTUM);
     bulk_prefetch_l2(Usrc + lam0 * E0, (uint32_t)nl * E0 * 8);
-    if (!draw) bulk_prefetch_l2(Qc + lam0 * E0, (uint32_t)nl * E0 * 8);
+    bulk_prefetch_l2(Qc + lam0 * E0, (uint32_t)nl * E0 * 8);
     bulk_prefetch_l2(v.sinv + lam0 * E0, (uint32_t)nl * E0 * 4);
   }
 
@@ -298,7 +549,6 @@ __global__ void __launch_bounds__(XCfg<E0>::NT, XCfg<E0>::MINB) k_xline(DevVolum
   const bool fixed = (flags & XF_FIXED_MOMENTUM) != 0;
   const bool write_q = !last || (flags & XF_WRITE_Q_LAST);
   const float keps = ((first || last) ? 0.5f : 1.0f) * eps;
-  const float Nf = (float)N;
   double pa = 0.0, pb = 0.0;
   for (int e = threadIdx.x; e < TL * (E0 / 2); e += NT) {
     const int l = e / (E0 / 2), x = 2 * (e % (E0 / 2));
@@ -306,17 +556,8 @@ __global__ void __launch_bounds__(XCfg<E0>::NT, XCfg<E0>::MINB) k_xline(DevVolum
     const long long gi = (lam0 + l) * E0 + x;
     const float4 u4 = __ldcs(reinterpret_cast<const float4*>(Usrc + gi));
     const float2 s2 = *reinterpret_cast<const float2*>(v.sinv + gi);
-    float4 q4;
-    float2 w0 = make_float2(0.f, 0.f), w1 = w0;
-    if (first && !fixed) {
-      const u32x4 r = philox(u32x4{(uint32_t)(gi >> 1), (uint32_t)st.iteration, (uint32_t)(ch.chain0 + c),
-                                   RNG_MOMENTUM}, ch.seed);
-      w0 = box_muller(u01f(r.x), u01f(r.y));
-      w1 = box_muller(u01f(r.z), u01f(r.w));
-      pa += (double)(w0.x * w0.x + w0.y * w0.y) + (double)(w1.x * w1.x + w1.y * w1.y);
-    } else {
-      q4 = __ldcs(reinterpret_cast<const float4*>(Qc + gi));
-    }
+    const float4 q4 = __ldcs(reinterpret_cast<const float4*>(Qc + gi));
+    const double wt = (first || last) ? plane_weight((int)((lam0 + l) / v.E1), v.E2) : 0.0;
     float2 uo[2], qo[2];
 #pragma unroll
     for (int m = 0; m < 2; m++) {
@@ -324,16 +565,11 @@ __global__ void __launch_bounds__(XCfg<E0>::NT, XCfg<E0>::MINB) k_xline(DevVolum
       const float s = m == 0 ? s2.x : s2.y;
       const bool live = s > 0.0f;
       const float lm = s + sh;  // lambda_m = 1/lambda + sigma_h^-2 (MultiResParameters.h:735-738)
-      float2 q;
-      if (first && !fixed) {
-        const float2 w = m == 0 ? w0 : w1;
-        const float a = live ? sqrtf(Nf * lm) : 0.0f;
-        q = make_float2(a * w.x, a * w.y);
-      } else {
-        q = m == 0 ? make_float2(q4.x, q4.y) : make_float2(q4.z, q4.w);
-        if (first && live) pa += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+      float2 q = m == 0 ? make_float2(q4.x, q4.y) : make_float2(q4.z, q4.w);
+      if (first && live) {  // the kinetic energy of a drawn momentum is k_momentum's sum |w|^2
+        if (fixed) pa += wt * ((double)(q.x * q.x + q.y * q.y) / (double)lm);
+        pb += wt * ((double)(u.x * u.x + u.y * u.y) * (double)s);
       }
-      if (first && live) pb += (double)(u.x * u.x + u.y * u.y) * (double)s;
       const float2 g = sm[(x + m) * P + l];
       float2 gt = g;
       if (live) {
@@ -347,8 +583,8 @@ __global__ void __launch_bounds__(XCfg<E0>::NT, XCfg<E0>::MINB) k_xline(DevVolum
         // the final energies; a step that is both first and last only evaluates (a gradient / log posterior
         // call) and keeps the energies at mu
         if (live && !first) {
-          pa += (double)(u.x * u.x + u.y * u.y) * (double)s;
-          pb += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+          pa += wt * ((double)(u.x * u.x + u.y * u.y) * (double)s);
+          pb += wt * ((double)(q.x * q.x + q.y * q.y) / (double)lm);
         }
       } else if (live) {
         const float f = eps / lm;
@@ -451,26 +687,23 @@ __device__ __forceinline__ void plane_fft(float2* sm, int ncols, int nrows, int 
   }
 }
 
-// One plane of one chain after its inverse transforms, in two parts.  plane_update: the kick (and at step 0 the
-// momentum draw) and the drift, with the state read from srcU / srcQ / srcS (global memory, or shared-memory copies
-// of this plane) and written to Udst / Qc in global memory; the energies' per-thread partials go to pa / pb.
-// need_q: the momentum is read (false only for the momentum draw at step 0).  GSRC: srcU / srcQ are in global
-// memory, read with streaming loads (ld.global.cs), as the U and q stores are made; a plane's state is not read
+// One plane of one chain after its inverse transforms, in two parts.  plane_update: the kick and the drift, with the
+// state read from srcU / srcQ / srcS (global memory, or shared-memory copies of this plane) and written to Udst / Qc
+// in global memory; the energies' per-thread partials go to pa / pb.  GSRC: srcU / srcQ are in global memory, read with streaming loads (ld.global.cs), as the U and q stores are made; a plane's state is not read
 // again before the next leapfrog step, by which time it has left L2 anyway, and evicting it first keeps T2 and the
 // smaller arrays of the following kernels in L2 (5.97 against 6.04 ms per 64-chain iteration).  The shared-memory
 // copies of the prefetching variant take plain loads: a global-space load of a shared address is an error.
 // plane_finish: the energies' block partials, then the forward transforms and the T2 store.
 template <int E, int NT, bool GSRC>
-__device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, const DevChains& ch,
-                                             const ChainState& st, int c, int z, bool first, bool last, bool need_q,
-                                             int flags, const float2* srcU, const float2* srcQ, const float* srcS,
+__device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, const ChainState& st, int z, bool first, bool last, int flags,
+                                             const float2* srcU, const float2* srcQ, const float* srcS,
                                              float2* Udst, float2* Qc, double& pa_out, double& pb_out) {
   using G = PlaneGeom<E>;
   const int tid = threadIdx.x;
   const float eps = st.eps_cur, sh = st.sh;
   const bool write_q = !last || (flags & XF_WRITE_Q_LAST);
   const float keps = ((first || last) ? 0.5f : 1.0f) * eps;
-  const float Nf = (float)v.N;
+  const bool fixed = (flags & XF_FIXED_MOMENTUM) != 0;
   double pa = 0.0, pb = 0.0;
   // Pairs of x-adjacent points: element pair e sits at li = 2e of the plane (x = 2 (e mod E/2), y = e / (E/2)),
   // so U, q and 1/lambda are read as float4 / float4 / float2 at index e.  Each thread issues the loads of B pairs
@@ -493,10 +726,10 @@ __device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, con
       if (e < TOTAL) {
         if constexpr (GSRC) {
           u4v[b] = __ldcs(gU + e);
-          q4v[b] = need_q ? __ldcs(gQ + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+          q4v[b] = __ldcs(gQ + e);
         } else {
           u4v[b] = gU[e];
-          q4v[b] = need_q ? gQ[e] : make_float4(0.f, 0.f, 0.f, 0.f);
+          q4v[b] = gQ[e];
         }
         s2v[b] = gS[e];
       }
@@ -509,15 +742,6 @@ __device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, con
       const float4 u4 = u4v[b];
       const float2 s2 = s2v[b];
       const float4 q4 = q4v[b];
-      float2 w0 = make_float2(0.f, 0.f), w1 = w0;
-      if (!need_q) {
-        const long long gi = (long long)z * E * E + 2 * e;
-        const u32x4 r = philox(u32x4{(uint32_t)(gi >> 1), (uint32_t)st.iteration, (uint32_t)(ch.chain0 + c),
-                                     RNG_MOMENTUM}, ch.seed);
-        w0 = box_muller(u01f(r.x), u01f(r.y));
-        w1 = box_muller(u01f(r.z), u01f(r.w));
-        pa += (double)(w0.x * w0.x + w0.y * w0.y) + (double)(w1.x * w1.x + w1.y * w1.y);
-      }
       const int pi0 = G::at(y, x), pi1 = pi0 + 1;  // x is even: x + 1 is the next slot in either layout
       float2 uo[2], qo[2];
 #pragma unroll
@@ -526,16 +750,11 @@ __device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, con
         const float s = m == 0 ? s2.x : s2.y;
         const bool live = s > 0.0f;
         const float lm = s + sh;
-        float2 q;
-        if (!need_q) {
-          const float2 w = m == 0 ? w0 : w1;
-          const float a = live ? sqrtf(Nf * lm) : 0.0f;
-          q = make_float2(a * w.x, a * w.y);
-        } else {
-          q = m == 0 ? make_float2(q4.x, q4.y) : make_float2(q4.z, q4.w);
-          if (first && live) pa += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+        float2 q = m == 0 ? make_float2(q4.x, q4.y) : make_float2(q4.z, q4.w);
+        if (first && live) {  // the kinetic energy of a drawn momentum is k_momentum's sum |w|^2
+          if (fixed) pa += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+          pb += (double)(u.x * u.x + u.y * u.y) * (double)s;
         }
-        if (first && live) pb += (double)(u.x * u.x + u.y * u.y) * (double)s;
         const int pi = m == 0 ? pi0 : pi1;
         const float2 g = sm[pi];
         float2 gt = g;
@@ -564,8 +783,9 @@ __device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, con
       if (!last) __stcs(oU + e, make_float4(uo[0].x, uo[0].y, uo[1].x, uo[1].y));
     }
   }
-  pa_out = pa;
-  pb_out = pb;
+  const double wt = plane_weight(z, v.E2);
+  pa_out = wt * pa;
+  pb_out = wt * pb;
 }
 
 template <int E, int NT>
@@ -624,20 +844,18 @@ __global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETC
   const int Lc = st.L_cur;
   if (step > Lc) return;
   // the block's plane of the state and of T2 lie in their arrays (checked builds)
-  if (!in_bounds((long long)(z + 1) * E * E - 1, v.N, ch.err) ||
+  if (!in_bounds((long long)(z + 1) * E * E - 1, v.NH, ch.err) ||
       !in_bounds((long long)(z + 1) * v.by * v.bx - 1, ch.t2_stride, ch.err))
     return;
   const bool first = step == 0, last = step == Lc;
-  const bool fixed = (flags & XF_FIXED_MOMENTUM) != 0;
-  const bool need_q = !(first && !fixed);
   const int acc = st.acc;
-  const long long N = v.N;
+  const long long NH = v.NH;
   const int bx = v.bx, by = v.by;
   const int tid = threadIdx.x;
-  float2* Ub = ch.U + (long long)c * 2 * N;
-  const float2* Usrc = Ub + (long long)(first ? acc : (acc ^ 1)) * N + (long long)z * E * E;
-  float2* Udst = Ub + (long long)(acc ^ 1) * N + (long long)z * E * E;
-  float2* Qc = ch.Q + (long long)c * N + (long long)z * E * E;
+  float2* Ub = ch.U + (long long)c * 2 * NH;
+  const float2* Usrc = Ub + (long long)(first ? acc : (acc ^ 1)) * NH + (long long)z * E * E;
+  float2* Udst = Ub + (long long)(acc ^ 1) * NH + (long long)z * E * E;
+  float2* Qc = ch.Q + (long long)c * NH + (long long)z * E * E;
   const float* Sg = v.sinv + (long long)z * E * E;
   float2* T = ch.T2 + (long long)c * ch.t2_stride + (long long)z * by * bx;
   // the twiddles of length E in shared memory: the row and column stages load a lane's twiddles again for every
@@ -650,7 +868,7 @@ __global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETC
   uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
   if (!PREFETCH && (flags & XF_L2_PREFETCH) && tid == 0) {
     bulk_prefetch_l2(Usrc, E * E * 8);
-    if (need_q) bulk_prefetch_l2(Qc, E * E * 8);
+    bulk_prefetch_l2(Qc, E * E * 8);
     bulk_prefetch_l2(Sg, E * E * 4);
   }
   if constexpr (PREFETCH) {
@@ -661,9 +879,9 @@ __global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETC
       mbar_init(bar, 1);
       mbar_fence_init();
       const uint32_t bu = E * E * 8;
-      mbar_arrive_expect_tx(bar, need_q ? 2 * bu : bu);
+      mbar_arrive_expect_tx(bar, 2 * bu);
       bulk_g2s(smraw + Ly.u_off, Usrc, bu, bar);
-      if (need_q) bulk_g2s(smraw + Ly.q_off, Qc, bu, bar);
+      bulk_g2s(smraw + Ly.q_off, Qc, bu, bar);
     }
   }
   plane_load_box<E, NT>(sm, T, bx, by);
@@ -680,7 +898,7 @@ __global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETC
     }
   }
   double pa, pb;
-  plane_update<E, NT, !PREFETCH>(sm, v, ch, st, c, z, first, last, need_q, flags, srcU, srcQ, Sg, Udst, Qc, pa, pb);
+  plane_update<E, NT, !PREFETCH>(sm, v, st, z, first, last, flags, srcU, srcQ, Sg, Udst, Qc, pa, pb);
   plane_finish<E, NT>(sm, ch, c, z, first, last, pa, pb, T, bx, by, twE, red);
 }
 
@@ -965,7 +1183,8 @@ __global__ void __launch_bounds__(256) k_accept(DevVolume v, DevChains ch) {
   const int c = blockIdx.x;
   ChainState& st = ch.st[c];
   if (st.L_cur < 0) return;
-  const int nbs[8] = {ch.nb_x, ch.nb_x, ch.nb_wt, ch.nb_w, ch.nb_x, ch.nb_x, ch.nb_wt, ch.nb_w};
+  const int ne = ch.nb_x + ch.nb_g;
+  const int nbs[8] = {ne, ne, ch.nb_wt, ch.nb_w, ne, ne, ch.nb_wt, ch.nb_w};
   for (int s = 0; s < 8; s++) {
     double t = 0.0;
     if (!((s == SL_RS0 || s == SL_RSL) && v.n_s == 0)) t = slot_sum(ch, c, s, nbs[s], red);
@@ -1081,26 +1300,29 @@ __global__ void k_fill_gD(DevVolume v, DevChains ch) {
 }
 
 // _initialize_mu (MultiResParameters.h:744-759) in the spectral basis:
-// u0 += sqrt(N lambda) w / 10 on live modes, w ~ CN(0, 2).
+// u0 += sqrt(N lambda) w / 10 on live modes, w ~ CN(0, 2) over all N modes, split into h and g as in k_momentum.
 __global__ void k_init_prior(DevVolume v, DevChains ch) {
-  const long long pair = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const int c = blockIdx.y;
-  if (2 * pair >= v.N) return;
-  const long long gi = 2 * pair;
-  float2* U = ch.U + (long long)c * 2 * v.N + (long long)ch.st[c].acc * v.N;
-  const u32x4 r = philox(u32x4{(uint32_t)pair, 0u, (uint32_t)(ch.chain0 + c), RNG_INIT_MU}, ch.seed);
-  const float2 w0 = box_muller(u01f(r.x), u01f(r.y)), w1 = box_muller(u01f(r.z), u01f(r.w));
-  const float Nf = (float)v.N;
-#pragma unroll
-  for (int m = 0; m < 2; m++) {
-    const float s = v.sinv[gi + m];
-    if (s > 0.0f) {
-      const float a = sqrtf(Nf / s) * 0.1f;
-      const float2 w = m == 0 ? w0 : w1;
-      U[gi + m].x += a * w.x;
-      U[gi + m].y += a * w.y;
-    }
+  if (i >= v.NH) return;
+  const int x = (int)(i % v.E0), y = (int)((i / v.E0) % v.E1), z = (int)(i / ((long long)v.E0 * v.E1));
+  const long long j = ((long long)(z == 0 ? 0 : v.E2 - z) * v.E1 + (y == 0 ? 0 : v.E1 - y)) * v.E0 + (x == 0 ? 0 : v.E0 - x);
+  const long long half = ((long long)c * 2 + ch.st[c].acc) * v.NH;
+  auto draw = [&](long long k) {
+    const u32x4 r = philox(u32x4{(uint32_t)(k >> 1), 0u, (uint32_t)(ch.chain0 + c), RNG_INIT_MU}, ch.seed);
+    return (k & 1) ? box_muller(u01f(r.z), u01f(r.w)) : box_muller(u01f(r.x), u01f(r.y));
+  };
+  const float s = v.sinv[i];
+  float2 g = make_float2(0.f, 0.f);
+  if (s > 0.0f) {
+    const float a = 0.5f * (sqrtf((float)v.N / s) * 0.1f);
+    const float2 w = draw(i), m = draw(j);
+    float2& h = ch.U[half + i];
+    h.x += a * (w.x + m.x);
+    h.y += a * (w.y - m.y);
+    g = make_float2(a * (w.y + m.y), a * (m.x - w.x));
   }
+  ch.G[half + i] = g;
 }
 
 // ----------------------------------------------------------------- spectrum (FP64, one-time)
@@ -1128,18 +1350,19 @@ __global__ void k_base(double2* base, int E0, int E1, int E2, float q00, float q
   base[i] = make_double2(val, 0.0);
 }
 
-// S = {Re lambda <= 0} (MultiResParameters.h:258-262); sinv = 1/Re lambda on live modes.
-__global__ void k_spectrum(const double2* lam, float* sinv, double* lam_re, long long N, int* n_S) {
+// S = {Re lambda <= 0} (MultiResParameters.h:258-262); sinv = 1/Re lambda on live modes.  The base is even in every
+// axis, so lambda(k) and lambda(-k) are the same number; the transform leaves them a rounding apart.  sinv is formed
+// from their mean, which both get bit for bit: a Hermitian field stays Hermitian under the sampler's element-wise
+// steps.  (lam_re and n_S report the transform's own values.)
+__global__ void k_spectrum(const double2* lam, float* sinv, double* lam_re, int E0, int E1, int E2, int* n_S) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= N) return;
-  const double re = lam[i].x;
+  if (i >= (long long)E0 * E1 * E2) return;
+  const int x = (int)(i % E0), y = (int)((i / E0) % E1), z = (int)(i / ((long long)E0 * E1));
+  const long long j = ((long long)(z == 0 ? 0 : E2 - z) * E1 + (y == 0 ? 0 : E1 - y)) * E0 + (x == 0 ? 0 : E0 - x);
+  const double re = lam[i].x, sym = 0.5 * (re + lam[j].x);
   lam_re[i] = re;
-  if (re > 0.0) {
-    sinv[i] = (float)(1.0 / re);
-  } else {
-    sinv[i] = -1.0f;
-    atomicAdd(n_S, 1);
-  }
+  if (re <= 0.0) atomicAdd(n_S, 1);
+  sinv[i] = sym > 0.0 ? (float)(1.0 / sym) : -1.0f;
 }
 
 // ----------------------------------------------------------------- evaluation helpers
