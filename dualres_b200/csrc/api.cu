@@ -748,8 +748,8 @@ struct Chainset {
   bool tcp = false;             // kriging products on the tensor cores (dense tiles of the volume)
   int tc_N = 0;                 // chains per tensor-core product (power of two >= C)
   float* tc_partial = nullptr;  // [segments][tc_N][128] partial products
-  bool tc_tg = false;           // W^T rs: the chain vectors arrive by TMA row gathers over tc_map_wt
-  CUtensorMap tc_map_w{}, tc_map_wt{};  // (tc_map_w unused: W mu_D gathers with its threads); rs as [n_s] rows
+  bool tc_tg = false;           // the chain vectors arrive by TMA row gathers over tc_map_w / tc_map_wt
+  CUtensorMap tc_map_w{}, tc_map_wt{};  // mu_D as [2 n_h] rows; rs as [n_s] rows
   bool tma = false;             // path 1
   int tma_smem = 0, tma_grid = 0;
 
@@ -854,9 +854,7 @@ static void launch_tc(Chainset* S, int step, int sel, int chain_only, bool w) {
     const size_t sm = tc_smem_bytes(N);
     const CUtensorMap& xm = w ? S->tc_map_w : S->tc_map_wt;
     float* P = S->tc_partial;
-    // TMA row gathers for W^T rs (one row set per chunk); W mu_D would need both halves of mu_D per chunk, twice
-    // the gathered bytes in twice the operations, and measured faster with the threads' own loads
-    const bool tg = S->tc_tg && !w;
+    const bool tg = S->tc_tg;
 #define DRB_TC_LAUNCH(NN)                                                                                 \
   if (tg) launch_k(k_tc_product<NN, true>, M.G, tc_threads(NN), sm, S->stream, M, S->dc, n_h, sel, mode, P, xm); \
   else launch_k(k_tc_product<NN, false>, M.G, tc_threads(NN), sm, S->stream, M, S->dc, n_h, sel, mode, P, xm);
@@ -992,7 +990,7 @@ static void enqueue_steps(Chainset* S, int L, int flags) {
   for (int s = 0; s <= L; s++) {
     const NvtxRange range(s == 0 ? "leapfrog step 0 (half kick, drift)"
                                  : (s == L ? "leapfrog last step (half kick, energies)" : "leapfrog step"));
-    const int sel = s == 0 ? 0 : 1;
+    const int sel = s == 0 && !(flags & XF_EVAL) ? 0 : 1;
     if (s > 0) {
       if (!S->plane) launch_y(S, -1, s);
       // forward z (pruned to the box), gather mu at data / output voxels
@@ -1020,7 +1018,7 @@ static void enqueue_iteration(Chainset* S) {
   CK_LAUNCH();
   k_summary_max<<<S->C, 256, 0, S->stream>>>(v, S->dc);
   CK_LAUNCH();
-  k_summary_acc<<<std::max(1, cdiv_i((long long)v.n_o * S->dc.Cp, 256)), 256, 0, S->stream>>>(v, S->dc);
+  k_summary_acc<<<std::max(1, cdiv_i((long long)std::max(v.n_o, v.n_h) * S->dc.Cp, 256)), 256, 0, S->stream>>>(v, S->dc);
   CK_LAUNCH();
 }
 
@@ -1437,14 +1435,18 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
     ch.nb_w = tc_finish_blocks(V->tc_w.T);
     ch.nb_wt = tc_finish_blocks(V->tc_wt.T);
     S->tc_partial = S->alloc<float>((size_t)std::max(V->tc_max_segs, 1) * S->tc_N * TC_M, false);
+    // TMA row gathers from 32 chains (rows of 128 bytes): 64 chains on a 32^3 volume W 23.7 / W^T 20.3 us against 25.0 /
+    // 20.9 with the threads' own loads, 16 chains on 64x64x48 61.3 / 46.2 against 58.0 / 45.2
     const char* tg = std::getenv("DRB_TC_TMA_GATHER");
-    S->tc_tg = !(tg && std::string(tg) == "0") && encode_row_map(&S->tc_map_wt, ch.rs, ch.Cp, (long long)v.n_s, S->tc_N);
+    S->tc_tg = !(tg && std::string(tg) == "0") && S->tc_N >= 32 && encode_row_map(&S->tc_map_wt, ch.rs, ch.Cp, (long long)v.n_s, S->tc_N) &&
+               encode_row_map(&S->tc_map_w, ch.muD, ch.Cp, 2LL * v.n_h, S->tc_N);
   }
   // k_momentum's row groups, at most four blocks per SM taking them in turn
   ch.nb_g = std::min(cdiv_i((long long)v.EZ * v.E1, MOM_ITEMS / v.E0), 592);
   ch.maxblk = std::max(ch.nb_x + ch.nb_g, std::max(ch.nb_w, ch.nb_wt));
   ch.part = S->alloc<double>((size_t)C * NSLOT * ch.maxblk);
   ch.st = S->alloc<ChainState>(C);
+  ch.moved = S->alloc<int>(C);
   ch.s1 = S->alloc<double>((size_t)std::max(v.n_o, 1) * C);
   ch.s2 = S->alloc<double>((size_t)std::max(v.n_o, 1) * C);
   ch.sa = S->alloc<double>((size_t)std::max(v.n_o, 1) * C);
@@ -1655,7 +1657,7 @@ static void eval_sampler(Chainset* S, int chain, const float* mu, double* lpll, 
   saved = st;
   const int half = st[chain].acc ^ 1;
   upload_field(S, mu);
-  gather_data(S, S->tmp, chain, half, false);
+  gather_data(S, S->tmp, chain, 1, false);
   forward_field(S, S->dc.U + state_off(S, chain, half), S->dc.G + state_off(S, chain, half));
   CK(cudaMemsetAsync(S->dc.Q + (long long)chain * v.NH, 0, sizeof(float2) * v.NH, S->stream));
   CK(cudaMemsetAsync(S->dc.Gq, 0, sizeof(float2) * v.NH, S->stream));
@@ -1665,7 +1667,7 @@ static void eval_sampler(Chainset* S, int chain, const float* mu, double* lpll, 
   st[chain].acc = half;
   write_states(S, st);
   try {
-    enqueue_steps(S, 0, XF_FIXED_MOMENTUM | XF_WRITE_Q_LAST);
+    enqueue_steps(S, 0, XF_FIXED_MOMENTUM | XF_WRITE_Q_LAST | XF_EVAL);
     if (lpll) {
       const double lp = part_sum(S, chain, SL_LP0, S->dc.nb_x + S->dc.nb_g);
       const double Rh = part_sum(S, chain, SL_RH0, S->dc.nb_wt);
@@ -1947,7 +1949,7 @@ int dr_set_state(dr_chainset* s, int chain, const float* mu, float s_hr, float s
   const DevVolume& v = s->vol->dv;
   const int acc = st[chain].acc;
   upload_field(s, mu);
-  gather_data(s, s->tmp, chain, acc, true);
+  gather_data(s, s->tmp, chain, 0, true);
   forward_field(s, s->dc.U + state_off(s, chain, acc), s->dc.G + state_off(s, chain, acc));
   st[chain].sh = s_hr;
   st[chain].ss = s_sr;
@@ -1956,8 +1958,8 @@ int dr_set_state(dr_chainset* s, int chain, const float* mu, float s_hr, float s
 }
 
 // Checkpoint layout: a header of eight int64 {magic, version, C, N, n_h, n_o, Cp, nsave_stored}, then per chain the
-// accepted spectral state (version 2: the half spectra of Re mu and Im mu, NH float2 each; version 1, still read: the
-// spectrum of mu, N float2), mu_D [2][n_h][Cp] and mu_O [2][n_o][Cp] floats, the ChainState array, the
+// accepted spectral state (from version 2: the half spectra of Re mu and Im mu, NH float2 each; version 1, still read:
+// the spectrum of mu, N float2; before version 3 the accepted half of mu_D and mu_O was half acc, not half 0), mu_D [2][n_h][Cp] and mu_O [2][n_o][Cp] floats, the ChainState array, the
 // summary sums s1, s2, sa [n_o][Cp] doubles, and with stored samples the samples [nsave][n_o][Cp] floats and the
 // sample records [nsave][C][3] doubles.
 struct CheckpointShape {
@@ -1975,7 +1977,7 @@ struct CheckpointShape {
     return b;
   }
 };
-static constexpr int64_t CKPT_MAGIC = 0x44524232434b5054LL, CKPT_VERSION = 2;
+static constexpr int64_t CKPT_MAGIC = 0x44524232434b5054LL, CKPT_VERSION = 3;
 
 static CheckpointShape checkpoint_shape(const Chainset* s) {
   const DevVolume& v = s->vol->dv;
@@ -2025,6 +2027,10 @@ static void checkpoint_copy(Chainset* s, unsigned char* buf, bool to_host, int64
   o = mu_off;
   copy(ch.muD, sizeof(float) * 2 * sh.n_h * sh.Cp, o);
   copy(ch.muO, sizeof(float) * 2 * no * sh.Cp, o);
+  if (!to_host && version < 3) {
+    k_adopt_halves<<<cdiv_i(std::max(sh.n_h, no) * sh.Cp, 256), 256, 0, st>>>(s->vol->dv, ch);
+    CK_LAUNCH();
+  }
   o = st_end;
   copy(ch.s1, sizeof(double) * no * sh.Cp, o);
   copy(ch.s2, sizeof(double) * no * sh.Cp, o);
@@ -2124,7 +2130,7 @@ int dr_leapfrog_fixed(dr_chainset* s, int chain, const float* mu0, const float* 
   const int acc = st[chain].acc;
   // u0 and the data values of mu0
   upload_field(s, mu0);
-  gather_data(s, s->tmp, chain, acc, false);
+  gather_data(s, s->tmp, chain, 0, false);
   forward_field(s, s->dc.U + state_off(s, chain, acc), s->dc.G + state_off(s, chain, acc));
   // q0 = IFFT(p0)
   upload_field(s, p0);

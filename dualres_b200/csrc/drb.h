@@ -35,7 +35,7 @@ struct ChainState {
   float eps_cur;   // step size used by this iteration
   int L_cur;       // leapfrog steps of this iteration; < 0 = chain idle
   float sh, ss;    // sigma_h^-2, sigma_s^-2
-  int acc;         // which half of U / muD / muO holds the accepted state
+  int acc;         // which half of U and G holds the accepted state
   int saved;       // samples saved
   int done;        // nsave reached
   int save_now;    // this iteration was a save iteration
@@ -83,8 +83,9 @@ struct DevChains {
   float2* T1;               // [C][EZ*E1*bx]
   float2* T2;               // [C][EZ*by*bx]
   long long t1_stride, t2_stride;
-  float* muD;               // [2][n_h][Cp] Re mu at data voxels
-  float* muO;               // [2][n_o][Cp] Re mu at output voxels
+  float* muD;               // [2][n_h][Cp] Re mu at data voxels: half 0 accepted, half 1 proposal
+  float* muO;               // [2][n_o][Cp] Re mu at output voxels, the same
+  int* moved;               // [C] the last transition was accepted
   float* gD;                // [n_h][Cp] data gradient
   float* rs;                // [n_s][Cp] Ys - W mu_D
   double* part;             // [C][NSLOT][maxblk]
@@ -146,7 +147,8 @@ struct ZArgs {
 // x-line kernel flags
 // XF_L2_PREFETCH: the update kernels ask L2 for their blocks' state (u, q, 1/lambda) at entry, so that its DRAM
 // latency overlaps the inverse transforms.
-enum XFlags : int { XF_FIXED_MOMENTUM = 1, XF_WRITE_Q_LAST = 2, XF_L2_PREFETCH = 4 };
+// XF_EVAL: step 0 takes mu_D from the proposal half (an evaluation leaves the accepted half as it is).
+enum XFlags : int { XF_FIXED_MOMENTUM = 1, XF_WRITE_Q_LAST = 2, XF_L2_PREFETCH = 4, XF_EVAL = 8 };
 // Transforms that a chain set's tuning may switch to the second radix plan (fft_smem PLAN 1), one bit each.
 enum FftPlanBits : int { FP_ZINV = 1, FP_ZFWD = 2, FP_XLINE = 4 };
 

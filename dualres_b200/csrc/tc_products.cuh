@@ -80,11 +80,11 @@ __host__ __device__ constexpr int tc_threads(int N) { return 32 * (2 + 4 * tc_gr
 __host__ __device__ inline int tc_stage_bytes(int N) { return 2 * TC_BLK * 4 + 2 * N * TC_KC * 4; }
 __host__ __device__ inline int tc_smem_bytes(int N) { return TC_HDR + tc_stages(N) * tc_stage_bytes(N); }
 
-// mode 0: X = mu_D (each chain's accepted half xor sel), mode 1: X = rs.  N: chains, a power of two in [16, 256].
+// mode 0: X = mu_D (its half sel), mode 1: X = rs.  N: chains, a power of two in [16, 256].
 // TG: the chain vectors of a chunk's columns arrive by TMA row gathers (tile::gather4 over xmap, a 2D map of X with
-// rows of Cp chains and a one-row box of N chains) issued by warp 0 into the stage's B blocks -- for mu_D both
-// halves, half 0 into the hi block and half 1 into the lo block; padding columns fetch row 0, which meets zero
-// columns of A -- and the gather groups only read them from shared memory.  Without TG the gather groups load them.
+// rows of Cp chains and a one-row box of N chains) issued by warp 0 into the stage's hi B block -- padding columns
+// fetch row 0, which meets zero columns of A -- and the gather groups only read them from shared memory.  Without TG
+// the gather groups load them.
 template <int N, bool TG>
 __global__ void __launch_bounds__(tc_threads(N), 1)
     k_tc_product(DevTcMatrix A, DevChains ch, int n_h, int sel, int mode, float* __restrict__ partial,
@@ -98,8 +98,6 @@ __global__ void __launch_bounds__(tc_threads(N), 1)
   uint64_t* acce = fullA + 13;
   uint64_t* done = fullA + 14;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tsm + 128);
-  long long* xoff = reinterpret_cast<long long*>(tsm + 256);
-  int* xhalf = reinterpret_cast<int*>(tsm + 2304);
   unsigned char* stage0 = tsm + TC_HDR;
   const int stages = tc_stages(N), sbytes = tc_stage_bytes(N);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -118,16 +116,7 @@ __global__ void __launch_bounds__(tc_threads(N), 1)
     mbar_fence_init();
   }
   constexpr int G = tc_groups(N);
-  for (int n = threadIdx.x; n < N; n += tc_threads(N)) {
-    long long o = -1;
-    int h = -1;
-    if (n < ch.C) {
-      h = mode == 0 ? (ch.st[n].acc ^ sel) : 0;
-      o = (long long)h * n_h * ch.Cp + n;
-    }
-    xoff[n] = o;
-    xhalf[n] = h;
-  }
+  const int xrow = mode == 0 ? sel * n_h : 0;  // row of X that holds column 0
   if (warp == 1) {
     tmem_alloc(tmem_slot, ncols);
     tmem_relinquish();
@@ -139,11 +128,10 @@ __global__ void __launch_bounds__(tc_threads(N), 1)
   bool ok = true;
 
   if (warp == 0) {
-    // the whole warp: lane 0 bulk-copies A, lanes 0-7 (and 8-15 for the second half of mu_D) gather 4 rows each.
+    // the whole warp: lane 0 bulk-copies A, lanes 0-7 gather 4 rows each.
     // A CTA's chunks are one contiguous range (its segments in order), and the column indices of the next chunk
     // are loaded while the current one is issued.
-    const int halves = mode == 0 ? 2 : 1;
-    const uint32_t xbytes = TG ? (uint32_t)halves * TC_KC * N * 4 : 0u;
+    const uint32_t xbytes = TG ? (uint32_t)TC_KC * N * 4 : 0u;
     const int c_begin = seg0 < seg1 ? A.segs[seg0].y : 0, c_end = seg0 < seg1 ? A.segs[seg1 - 1].z : 0;
     int jn = 0;
     if constexpr (TG) {
@@ -167,13 +155,12 @@ __global__ void __launch_bounds__(tc_threads(N), 1)
       }
       if constexpr (TG) {
         __syncwarp();
-        const int h = lane >> 3, r4 = (lane & 7) * 4;
+        const int r4 = (lane & 7) * 4;
         const int y0 = __shfl_sync(0xffffffffu, j, r4), y1 = __shfl_sync(0xffffffffu, j, r4 + 1);
         const int y2 = __shfl_sync(0xffffffffu, j, r4 + 2), y3 = __shfl_sync(0xffffffffu, j, r4 + 3);
-        if (h < halves) {
-          const int ro = h * n_h;
-          unsigned char* dst = stage0 + s * sbytes + 2 * TC_BLK * 4 + h * N * TC_KC * 4 + r4 * N * 4;
-          tma_gather4(dst, &xmap, 0, y0 + ro, y1 + ro, y2 + ro, y3 + ro, fullA + s);
+        if (lane < 8) {
+          unsigned char* dst = stage0 + s * sbytes + 2 * TC_BLK * 4 + r4 * N * 4;
+          tma_gather4(dst, &xmap, 0, y0 + xrow, y1 + xrow, y2 + xrow, y3 + xrow, fullA + s);
         }
       }
     }
@@ -249,7 +236,7 @@ __global__ void __launch_bounds__(tc_threads(N), 1)
         float4* bl = bh + N * (TC_KC / 4);
         float xv[NI][4];
         if constexpr (TG) {
-          // A and the gathered rows have landed: row k of half h at float h * 32N + k * N of the B blocks
+          // A and the gathered rows have landed: row k at float k * N of the hi B block
           got = got && mbar_wait_bounded(fullA + s, (q / stages) & 1);
           if (got) {
             const float* xs = reinterpret_cast<const float*>(bh);
@@ -257,10 +244,9 @@ __global__ void __launch_bounds__(tc_threads(N), 1)
             for (int i = 0; i < NI; i++) {
               const int idx = t + 128 * i;
               const int n = idx & (N - 1), kc4 = idx / N;
-              const int h = xhalf[n];
-              const float* r = xs + (h > 0 ? h : 0) * N * TC_KC + 4 * kc4 * N + n;
+              const float* r = xs + 4 * kc4 * N + n;
 #pragma unroll
-              for (int kk = 0; kk < 4; kk++) xv[i][kk] = h >= 0 ? r[kk * N] : 0.f;
+              for (int kk = 0; kk < 4; kk++) xv[i][kk] = n < ch.C ? r[kk * N] : 0.f;
             }
           }
           // every thread of the group has read the staged rows before the blocks are overwritten, and the group
@@ -280,9 +266,9 @@ __global__ void __launch_bounds__(tc_threads(N), 1)
           for (int i = 0; i < NI; i++) {
             const int idx = t + 128 * i;
             const int n = idx & (N - 1), kc4 = idx / N;
-            const long long o = xoff[n];
+            const long long o = xrow * Cp + n;
             const int4 j = __ldg(cols + kc4);
-            const bool on = o >= 0;
+            const bool on = n < ch.C;
             xv[i][0] = (on && j.x >= 0 && in_bounds(j.x, A.n_cols, ch.err)) ? __ldg(X + o + j.x * Cp) : 0.f;
             xv[i][1] = (on && j.y >= 0 && in_bounds(j.y, A.n_cols, ch.err)) ? __ldg(X + o + j.y * Cp) : 0.f;
             xv[i][2] = (on && j.z >= 0 && in_bounds(j.z, A.n_cols, ch.err)) ? __ldg(X + o + j.z * Cp) : 0.f;
@@ -424,7 +410,7 @@ __global__ void __launch_bounds__(256) k_tc_finish(DevTcMatrix A, const float* _
       }
     } else {
       const ChainState& st = ch.st[n];
-      const float* mu = ch.muD + (long long)(st.acc ^ sel) * v.n_h * Cp + n;
+      const float* mu = ch.muD + (long long)sel * v.n_h * Cp + n;
       const float sh = st.sh, ss = st.ss;
       float y[EPT], mv[EPT];
 #pragma unroll

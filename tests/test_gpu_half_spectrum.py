@@ -57,8 +57,9 @@ def test_gradient_and_leapfrog(oracle, monkeypatch, dims, dual, chains, ztile, l
 
 
 def test_checkpoint_of_the_full_spectrum_is_still_read():
-    """A version-1 checkpoint holds each chain's spectrum u = N IFFT(mu) on all N modes; restoring it gives the state
-    it was written from, to the rounding of one split."""
+    """A version-1 checkpoint holds each chain's spectrum u = N IFFT(mu) on all N modes, and the accepted mu at the
+    data and output voxels in either half (here in both); restoring it gives the state it was written from, to the
+    rounding of one split, and the fit goes on as the other one does."""
     vol = synth.small_volume(seed=9, dims=(9, 8, 6))
     data = d.MultiResData.from_volume(vol)
     hmc = d.HMCParameters(burnin=4, nsave=4, thin=1, leapfrog=3, seed=2)
@@ -67,17 +68,23 @@ def test_checkpoint_of_the_full_spectrum_is_still_read():
     ck = a.checkpoint()
     head = np.frombuffer(ck[:64], np.int64).copy()
     nh = data.N // data.shape[0] * (data.shape[0] // 2 + 1)
-    assert head[1] == 2 and head[3] == data.N
+    assert head[1] == 3 and head[3] == data.N
     head[1] = 1
     u = [(np.fft.ifftn(a.get_state(c)[0].astype(np.complex128)) * data.N).astype(np.complex64) for c in range(2)]
-    old = head.tobytes() + b"".join(x.tobytes() for x in u) + ck[64 + 2 * 2 * nh * 8:]
+    at = 64 + 2 * 2 * nh * 8
+    halves = []
+    for n in (data.n_highres, data.n_output):
+        mu = ck[at:at + n * 2 * 4]
+        halves.append(mu + mu)
+        at += 2 * len(mu)
     b = d.MultiResParameters(data, hmc, 2)
-    b.restore(old)
-    for c in range(2):
-        (mu, s), (want, t) = b.get_state(c), a.get_state(c)
-        assert rel(mu, want) < 1e-6 and tuple(s) == tuple(t)
-    b.update(2)
-    head[1] = 3
+    b.restore(head.tobytes() + b"".join(x.tobytes() for x in u) + b"".join(halves) + ck[at:])
+    for steps in (0, 2):
+        a.update(steps), b.update(steps)
+        for c in range(2):
+            (mu, s), (want, t) = b.get_state(c), a.get_state(c)
+            assert rel(mu, want) < (1e-4 if steps else 1e-6) and np.allclose(s, t, rtol=1e-4)
+    head[1] = 4
     with pytest.raises(d.api.DrError):
         b.restore(head.tobytes() + ck[64:])
     a.close(), b.close(), data.close()
