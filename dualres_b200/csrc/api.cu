@@ -26,6 +26,7 @@
 #include "../../include/dualres_b200.h"
 #include "host_setup.h"
 #include "kernels.cu"
+#include "row_products.cuh"
 #include "tc_products.cuh"
 #include "mce.cuh"
 #include "kriging.cuh"
@@ -375,6 +376,8 @@ struct Volume {
   int64_t bytes = 0;
   const float2* tw_f = nullptr;
   const double2* tw_d = nullptr;
+  DevRowGroups rows_w{}, rows_wt{};  // row groups of W and W^T
+  int nb_w1 = 1, nb_wt1 = 1;  // blocks of the one-chain products (allocation-free evaluation)
   // Dense-tile form of W and W^T for the tensor-core products, built on first use by a chain set that can use
   // it (tc_state 0: not built, 1: built, -1: unavailable).
   std::mutex tc_mtx;
@@ -411,6 +414,9 @@ struct Volume {
 
 static std::mutex g_vol_mtx;
 
+// Blocks per SM of the row-group products of an untuned chain set (fewer where fewer are resident).
+constexpr int ROWP_BPS = 8;
+static int rowp_blocks(const DevRowGroups& M, const DevVolume& v, const DevChains& ch, bool w, int sms, int blocks_per_sm);
 
 // Kriging weights of a prepared volume on the device (k_kriging_rows), then
 // the CSR, its transpose and the host copies.  Rows whose system is not
@@ -641,6 +647,25 @@ static void kriging_solve_device(HostVolume& hv, int device, cudaStream_t st) {
   hv.kriging_seconds += dt_s;
 }
 
+// A matrix's row groups on the device.
+static void volume_rows(Volume* V, const std::vector<int>& rowptr, const int* col, const float* val, int n_cols,
+                        DevRowGroups* M) {
+  if (rowptr.size() < 2 || V->dv.n_s == 0) return;
+  const TraceScope tr("row groups");
+  RowGroupsHost h;
+  if (!row_groups(rowptr, col, val, &h)) throw Error(DR_ERR_UNSUPPORTED, "kriging matrix too large");
+  DevRowGroups& d = *M;
+  d.n_rows = (int)rowptr.size() - 1;
+  d.n_cols = n_cols;
+  d.groups = h.groups();
+  d.entries = (long long)h.off.size();
+  d.ptr = V->upload(h.ptr);
+  d.base = V->upload(h.base);
+  d.off = V->upload(h.off);
+  d.val = V->upload(h.val);
+  CK(cudaStreamSynchronize(V->stream));  // the host arrays are released on return
+}
+
 // Device part of a volume from an already prepared HostVolume (V->hv).
 static void volume_build_device(Volume* V, const float* covariance, int covfun, int device) {
   const NvtxRange range("volume: device set-up (kriging solves, FP64 spectrum)");
@@ -667,12 +692,16 @@ static void volume_build_device(Volume* V, const float* covariance, int covfun, 
   dv.o_flat = V->upload(hv.o_flat);
   dv.Yh = V->upload(hv.Yh);
   dv.Ys = V->upload(hv.Ys);
-  dv.w_rowptr = V->upload(hv.w_rowptr.empty() ? std::vector<int>{0} : hv.w_rowptr);
-  dv.w_col = V->upload(hv.w_col);
-  dv.w_val = V->upload(hv.w_val);
-  dv.wt_rowptr = V->upload(hv.wt_rowptr);
-  dv.wt_col = V->upload(hv.wt_col);
-  dv.wt_val = V->upload(hv.wt_val);
+  volume_rows(V, hv.w_rowptr, hv.w_col.data(), hv.w_val.data(), dv.n_h, &V->rows_w);
+  volume_rows(V, hv.wt_rowptr, hv.wt_col.data(), hv.wt_val.data(), dv.n_s, &V->rows_wt);
+  // W and W^T stay in L2 between the steps while they take less than half of it
+  V->rows_w.stream = V->rows_wt.stream = (V->rows_w.entries + V->rows_wt.entries) * 18 > (64LL << 20);
+  if (dv.n_s > 0) {
+    DevChains one{};
+    one.C = 1;
+    V->nb_w1 = rowp_blocks(V->rows_w, dv, one, true, dt.sms, ROWP_BPS);
+    V->nb_wt1 = rowp_blocks(V->rows_wt, dv, one, false, dt.sms, ROWP_BPS);
+  }
 
   // eigenvalues in FP64: base -> 3 forward passes -> S, 1/lambda
   const long long N = hv.N;
@@ -740,7 +769,7 @@ struct Chainset {
   int64_t graph_nodes = 0;
   std::vector<void*> allocs;
   float2* tmp = nullptr;        // [N] scratch for evaluation calls
-  int NR = 1;
+  int sms = 148;
   bool plane = false;           // fused xy-plane update (E0 == E1 <= 128)
   int path = 0;                 // 0 plane kernel, 1 plane kernel with bulk prefetch, 2 x-line kernel + y passes
   int grid = 8;                 // kriging-product blocks per SM
@@ -803,45 +832,82 @@ static void volume_release(Volume* v) {
   delete v;
 }
 
-template <int CG, int NR>
-static void launch_spmv_t(const DevVolume& v, const DevChains& ch, int nb, int step, int sel, int chain_only, bool w,
-                          cudaStream_t s) {
-  // a block per row while a block gets few rows; with at most 8 chains per warp, a warp per row once a block would
-  // take 8 or more of them in turn
-  bool rows = false;
-  if constexpr (CG <= 8) rows = w && v.n_s >= 8 * nb;
-  if (rows) {
-    if constexpr (CG <= 8) launch_k(k_spmv_w_rows<CG, NR>, nb, 256, 0, s, v, ch, step, sel, chain_only);
-  } else if (w) {
-    launch_k(k_spmv_w<CG, NR>, nb, 256, 0, s, v, ch, step, sel, chain_only);
-  } else
-    launch_k(k_spmv_wt<CG, NR>, nb, 256, 0, s, v, ch, step, sel, chain_only);
+struct RowpLaunch {
+  const DevVolume& v;
+  const DevRowGroups& M;
+  const DevChains& ch;
+  int nb, step, sel, chain_only;
+  int warps;  // per group
+  bool w;
+  cudaStream_t s;
+  int* resident;  // not null: report the blocks that fit an SM instead of launching
+};
+template <int V, int CL, int NR, int SW, bool WT>
+static void launch_rowp_k(const RowpLaunch& a) {
+  if (a.resident)
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(a.resident, k_row_product<V, CL, NR, SW, WT>, ROWP_NT, 0));
+  else
+    launch_k(k_row_product<V, CL, NR, SW, WT>, a.nb, ROWP_NT, 0, a.s, a.v, a.M, a.ch, a.step, a.sel, a.chain_only);
+}
+template <int V, int CL, int NR>
+static void launch_rowp_t(const RowpLaunch& a) {
+  if (!a.w) launch_rowp_k<V, CL, NR, 1, true>(a);
+  else if (a.warps == 8) launch_rowp_k<V, CL, NR, 8, false>(a);
+  else launch_rowp_k<V, CL, NR, 4, false>(a);
+}
+// CL lanes of V chains (the largest vector that divides C; up to 4 chains: a lane per entry with all of them, 3 chains in
+// 4 lanes) and NR rounds cover the chains.
+template <int V>
+static void launch_rowp_v(const RowpLaunch& a) {
+  const int lanes = a.ch.C / V;
+  if (lanes <= 1) return launch_rowp_t<V, 1, 1>(a);
+  if constexpr (V == 4)
+    if (lanes <= 2) return launch_rowp_t<V, 2, 1>(a);
+  if (lanes <= 4) return launch_rowp_t<V, 4, 1>(a);
+  if (lanes <= 8) return launch_rowp_t<V, 8, 1>(a);
+  if (lanes <= 16) return launch_rowp_t<V, 16, 1>(a);
+  if (lanes <= 32) return launch_rowp_t<V, 32, 1>(a);
+  if (lanes <= 64) return launch_rowp_t<V, 32, 2>(a);
+  if constexpr (V <= 2)
+    if (lanes <= 128) return launch_rowp_t<V, 32, 4>(a);
+  if constexpr (V == 1) return launch_rowp_t<V, 32, 8>(a);
+}
+static void launch_rowp(const RowpLaunch& a) {
+  if (a.ch.C % 4 == 0) launch_rowp_v<4>(a);
+  else if (a.ch.C % 2 == 0) launch_rowp_v<2>(a);
+  else launch_rowp_v<1>(a);
+}
+// Warps that share a group: one for W^T; for W 8 with up to 2 chains per lane or when the groups are fewer than 8 per SM,
+// else 4 (2 chains, 80x80x64: 60 us with 8, 81 with 4; 12 chains, 281 groups: 9.7 and 13.9; 16 chains, 3294 groups: 36.4
+// and 30.7).
+static int rowp_warps(const DevRowGroups& M, const DevChains& ch, bool w, int sms) {
+  if (!w) return 1;
+  return (ch.C % 4 != 0 || M.groups < 8 * sms) ? 8 : 4;
+}
+// Blocks of a product: at most blocks_per_sm, and no more than are resident together, on every SM.
+static int rowp_blocks(const DevRowGroups& M, const DevVolume& v, const DevChains& ch, bool w, int sms, int blocks_per_sm) {
+  int fit = 1;
+  const int sw = rowp_warps(M, ch, w, sms);
+  launch_rowp(RowpLaunch{v, M, ch, 0, 0, 0, 0, sw, w, nullptr, &fit});
+  return std::max(1, std::min(cdiv_i(M.groups, 8 / sw), sms * std::min(blocks_per_sm, std::max(fit, 1))));
+}
+// Kriging products for the chains of `ch` from W's row groups (w) or W^T's.
+static void launch_rows(const DevVolume& v, const DevRowGroups& M, const DevChains& ch, int sms, int step, int sel,
+                        int chain_only, bool w, cudaStream_t s) {
+  const int nb = w ? ch.nb_w : ch.nb_wt;
+  if (nb > ch.maxblk || ch.part == nullptr) throw Error(DR_ERR_STATE, "partial-sum buffer smaller than the block count");
+  if (v.n_s == 0) {
+    int cw = 1;
+    while (cw < ch.C) cw *= 2;
+    launch_k(k_data_gradient, nb, ROWP_NT, 0, s, v, ch, cw, step, sel, chain_only);
+  } else {
+    launch_rowp(RowpLaunch{v, M, ch, nb, step, sel, chain_only, rowp_warps(M, ch, w, sms), w, s, nullptr});
+  }
   CK_LAUNCH();
 }
 
-// Kriging products for `ch` (chain group width CG = ch.CG, rounds NR).
-static void launch_spmv_dc(const DevVolume& v, const DevChains& ch, int NR, int step, int sel, int chain_only, bool w,
-                           cudaStream_t s) {
-  const int nb = w ? std::max(1, std::min(v.n_s, ch.nb_w)) : std::max(1, std::min(cdiv_i(v.n_h, 8), ch.nb_wt));
-  if (nb > ch.maxblk || ch.part == nullptr) throw Error(DR_ERR_STATE, "partial-sum buffer smaller than the block count");
-  switch (ch.CG) {
-    case 1: launch_spmv_t<1, 1>(v, ch, nb, step, sel, chain_only, w, s); break;
-    case 2: launch_spmv_t<2, 1>(v, ch, nb, step, sel, chain_only, w, s); break;
-    case 4: launch_spmv_t<4, 1>(v, ch, nb, step, sel, chain_only, w, s); break;
-    case 8: launch_spmv_t<8, 1>(v, ch, nb, step, sel, chain_only, w, s); break;
-    case 16: launch_spmv_t<16, 1>(v, ch, nb, step, sel, chain_only, w, s); break;
-    default:
-      switch (NR) {
-        case 1: launch_spmv_t<32, 1>(v, ch, nb, step, sel, chain_only, w, s); break;
-        case 2: launch_spmv_t<32, 2>(v, ch, nb, step, sel, chain_only, w, s); break;
-        case 4: launch_spmv_t<32, 4>(v, ch, nb, step, sel, chain_only, w, s); break;
-        default: launch_spmv_t<32, 8>(v, ch, nb, step, sel, chain_only, w, s); break;
-      }
-  }
-}
-
 // W mu_D (w) or W^T rs on the tensor cores: the tile products into segment partials, then the per-tile sums and
-// the same epilogue as the CSR kernels.
+// the same epilogue as the row-group kernels.
 static void launch_tc(Chainset* S, int step, int sel, int chain_only, bool w) {
   const Volume* V = S->vol;
   const DevTcMatrix& M = w ? V->tc_w : V->tc_wt;
@@ -882,7 +948,7 @@ static void launch_tc(Chainset* S, int step, int sel, int chain_only, bool w) {
 
 static void launch_spmv(Chainset* S, int step, int sel, int chain_only, bool w) {
   if (S->tcp) launch_tc(S, step, sel, chain_only, w);
-  else launch_spmv_dc(S->vol->dv, S->dc, S->NR, step, sel, chain_only, w, S->stream);
+  else launch_rows(S->vol->dv, w ? S->vol->rows_w : S->vol->rows_wt, S->dc, S->sms, step, sel, chain_only, w, S->stream);
 }
 
 // The update kernels' L2 prefetch of their state (XF_L2_PREFETCH); DRB_L2_PREFETCH=0 turns it off.
@@ -1061,7 +1127,7 @@ static void init_chain_states(Chainset* S) {
 // planes whose padded layout fits shared memory), the same with bulk prefetch
 // of the state planes, and the x-line kernel with separate y passes (always).
 // ---------------------------------------------------------------- tensor-core kriging products
-static void tc_upload(Volume* V, const TcPlanHost& P, const float* dval, int nnz, int n_rows, int n_cols,
+static void tc_upload(Volume* V, const TcPlanHost& P, const float* val, int nnz, int n_rows, int n_cols,
                       DevTcMatrix* M) {
   cudaStream_t st = V->stream;
   M->n_rows = n_rows;
@@ -1079,10 +1145,13 @@ static void tc_upload(Volume* V, const TcPlanHost& P, const float* dval, int nnz
   float* blob = V->alloc<float>(nblob);
   CK(cudaMemsetAsync(blob, 0, sizeof(float) * std::max<size_t>(nblob, 1), st));
   if (nnz > 0) {
+    // {position, value} of every nonzero, for the scatter only
     int* dest = nullptr;
-    const cudaError_t e = dev_alloc((void**)&dest, sizeof(int) * nnz, st);
+    const cudaError_t e = dev_alloc((void**)&dest, 2 * sizeof(int) * nnz, st);
     if (e != cudaSuccess) throw Error(DR_ERR_NOMEM, "device allocation (tile positions)");
+    float* dval = reinterpret_cast<float*>(dest + nnz);
     CK(cudaMemcpyAsync(dest, P.dest.data(), sizeof(int) * nnz, cudaMemcpyHostToDevice, st));
+    CK(cudaMemcpyAsync(dval, val, sizeof(float) * nnz, cudaMemcpyHostToDevice, st));
     k_tc_fill<<<cdiv_i(nnz, 256), 256, 0, st>>>(dval, dest, nnz, blob);
     CK_LAUNCH();
     CK(cudaFreeAsync(dest, st));
@@ -1139,8 +1208,8 @@ static bool volume_tc(Volume* V) {
   const double blob_bytes = (double)(pw.chunks + pt.chunks) * TC_BLK * 4;
   if (blob_bytes > 0.25 * (double)fr) return false;
   tr.next("tensor-core tiles: blob build");
-  tc_upload(V, pw, dv.w_val, (int)hv.w_col.size(), dv.n_s, dv.n_h, &V->tc_w);
-  tc_upload(V, pt, dv.wt_val, (int)hv.wt_col.size(), dv.n_h, dv.n_s, &V->tc_wt);
+  tc_upload(V, pw, hv.w_val.data(), (int)hv.w_col.size(), dv.n_s, dv.n_h, &V->tc_w);
+  tc_upload(V, pt, hv.wt_val.data(), (int)hv.wt_col.size(), dv.n_h, dv.n_s, &V->tc_wt);
   V->tc_max_segs = std::max(V->tc_w.n_segs, V->tc_wt.n_segs);
   CK(cudaStreamSynchronize(V->stream));
   V->tc_seconds = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
@@ -1206,7 +1275,7 @@ static PathOptions path_options(const DevVolume& v, int device) {
 struct TuneChoice {
   int ztile = 8;     // chains per z-pass tile (8 or 1) for chain sets of 8 or more chains
   int path = 0;      // 0 plane, 1 plane + prefetch, 2 x-line
-  int grid = 8;      // kriging-product blocks per SM (CSR products)
+  int grid = 8;      // kriging-product blocks per SM (row-group products)
   double ms = 0.0;   // measured milliseconds per iteration
   int tc = 0;        // 1: kriging products on the tensor cores
   int fftplan = 0;   // FP_* bits: transforms on the second radix plan (fft_smem PLAN 1) for 64, 128, 256 points
@@ -1241,8 +1310,8 @@ static int tune_bucket(int n) { return n <= 0 ? -1 : (int)std::lround(4.0 * std:
 // timed for one iteration after one untimed, forced past the step-size search
 // (so that all of their leapfrog steps run, at most 6 of them): first the update paths, with
 // the tensor-core products where the volume and chain count allow them (else
-// CSR products at 8 blocks per SM); then, on the fastest path, the other
-// product choices (CSR at 8 blocks/SM, and at 4 and 2 for chain sets of fewer
+// row-group products at 8 blocks per SM); then, on the fastest path, the other
+// product choices (row groups at 8 blocks/SM, and at 4 and 2 for chain sets of fewer
 // than 32 chains) and the z-pass tile shape.  The fastest candidate is kept
 // and cached per shape.
 static TuneChoice autotune(Volume* V, int C, const dr_hmc_opts* o) {
@@ -1309,7 +1378,7 @@ static TuneChoice autotune(Volume* V, int C, const dr_hmc_opts* o) {
   if (best.ms < 1e300) {
     const int path = best.path;
     if (tc) try_candidate(TuneChoice{8, path, 8, 0.0, 0});
-    // narrower chain sets may do better with fewer, longer-lived CSR product blocks
+    // narrower chain sets may do better with fewer, longer-lived product blocks
     if (C < 32)
       for (int grid : {4, 2}) try_candidate(TuneChoice{8, path, grid, 0.0, 0});
     // the z passes' tile shape on the best configuration: 32 lines of one chain instead of 4 lines x 8 chains
@@ -1360,13 +1429,7 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   DevChains& ch = S->dc;
   ch.C = C;
   ch.Cp = C;
-  int cg = 1;
-  while (cg < C && cg < 32) cg <<= 1;
-  ch.CG = cg;
-  S->NR = cdiv_i(C, cg);
-  if (S->NR > 8) throw Error(DR_ERR_UNSUPPORTED, "too many chains");
-  if (S->NR == 3) S->NR = 4;
-  if (S->NR > 4 && S->NR < 8) S->NR = 8;
+  S->sms = device_tables(V->device).sms;
   const long long N = v.N, NH = v.NH;
   const PathOptions po = path_options(v, V->device);
   int path = po.plane ? 0 : 2, grid = 8;
@@ -1426,9 +1489,6 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   ch.gD = S->alloc<float>((size_t)v.n_h * C);
   ch.rs = S->alloc<float>((size_t)std::max(v.n_s, 1) * C);
   ch.nb_x = S->plane ? v.EZ : cdiv_i((long long)v.E1 * v.EZ, TILE_LINES);
-  const int wide = device_tables(V->device).sms * S->grid;
-  ch.nb_w = std::max(1, std::min(v.n_s, wide));
-  ch.nb_wt = std::max(1, std::min(cdiv_i(v.n_h, 8), wide));
   S->tcp = tc && tc_chains(C) > 0 && volume_tc(V);
   if (S->tcp) {
     S->tc_N = tc_chains(C);
@@ -1440,6 +1500,14 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
     const char* tg = std::getenv("DRB_TC_TMA_GATHER");
     S->tc_tg = !(tg && std::string(tg) == "0") && S->tc_N >= 32 && encode_row_map(&S->tc_map_wt, ch.rs, ch.Cp, (long long)v.n_s, S->tc_N) &&
                encode_row_map(&S->tc_map_w, ch.muD, ch.Cp, 2LL * v.n_h, S->tc_N);
+  } else {
+    if (v.n_s > 0) {
+      ch.nb_w = rowp_blocks(V->rows_w, v, ch, true, S->sms, S->grid);
+      ch.nb_wt = rowp_blocks(V->rows_wt, v, ch, false, S->sms, S->grid);
+    } else {
+      ch.nb_w = 1;
+      ch.nb_wt = std::max(1, std::min(cdiv_i((long long)v.n_h * C, ROWP_NT), S->sms * 8));
+    }
   }
   // k_momentum's row groups, at most four blocks per SM taking them in turn
   ch.nb_g = std::min(cdiv_i((long long)v.EZ * v.E1, MOM_ITEMS / v.E0), 592);
@@ -2255,7 +2323,8 @@ int dr_debug_time_kernel(dr_chainset* s, int which, int stp, int reps, double* a
   const DevChains& ch = s->dc;
   const float2* tw = s->vol->tw_f;
   const int C = s->C;
-  const double NH = (double)v.NH, t1 = (double)ch.t1_stride, t2 = (double)ch.t2_stride, z = (double)s->vol->hv.w_col.size();
+  const double NH = (double)v.NH, t1 = (double)ch.t1_stride, t2 = (double)ch.t2_stride;
+  auto rows_bytes = [](const DevRowGroups& M) { return (double)M.entries * (4 * ROWP_R + 2 + 4.0 / 32) + M.groups * 4.0; };
   auto launch = [&]() {
     switch (which) {
       case 0: if (s->plane) launch_plane(s, stp, 0); else launch_xline(s, stp, 0); break;
@@ -2289,9 +2358,9 @@ int dr_debug_time_kernel(dr_chainset* s, int which, int stp, int reps, double* a
       case 0: b = C * (2.0 * (s->plane ? t2 : t1) * 8 + 4.0 * NH * 8) + NH * 4; break;  // T in/out, U and q in/out, 1/lambda
       case 1: b = s->plane ? 0.0 : C * (t1 + t2) * 8; break;
       case 2: b = C * (t2 * 8 + (v.n_h + v.n_o) * 4.0) + box * 8; break;            // box maps (2 x int32)
-      case 3: b = z * 8 + C * ((double)v.n_h * 4 + (double)v.n_s * 4) + v.n_s * 8.0; // W values + columns, mu_D, rs
-        break;
-      case 4: b = z * 8 + C * ((double)v.n_s * 4 + 2.0 * v.n_h * 4) + v.n_h * 12.0; break;
+      // the row groups' values, offsets, batch bases and pointers, the chain vectors, the data
+      case 3: b = rows_bytes(s->vol->rows_w) + C * ((double)v.n_h * 4 + (double)v.n_s * 4) + v.n_s * 4.0; break;
+      case 4: b = rows_bytes(s->vol->rows_wt) + C * ((double)v.n_s * 4 + 2.0 * v.n_h * 4) + v.n_h * 4.0; break;
       case 5: b = C * ((double)v.n_h * 4 + t2 * 8) + box * 4; break;
       default: b = s->plane ? 0.0 : C * (t2 + t1) * 8; break;
     }
@@ -2427,7 +2496,7 @@ static int64_t estimate_bytes(const HostVolume& hv, int C, const dr_hmc_opts& o)
   const double nh = (double)hv.Yh.size(), ns = (double)hv.Ys.size(), no = (double)hv.o_flat.size();
   const double nnz = (double)hv.w_col.size();
   const double ez = hv.E[2] / 2 + 1, NH = ez * hv.E[1] * hv.E[0], t2 = ez * hv.box[1] * hv.box[0];
-  double vol = box * 8 + (nh + no) * 4 + (nh + ns) * 4 + (ns + nh + 2) * 4 + nnz * 16 + N * 12 + N * 16;
+  double vol = box * 8 + (nh + no) * 4 + (nh + ns) * 4 + (ns + nh + 2) * 12 + nnz * (2.4 + 1.8) * 18 / 4 + N * 12 + N * 16;
   double cs = C * (5 * NH * 8 + t2 * 8 + (hv.E[0] == hv.E[1] ? 0.0 : ez * hv.E[1] * hv.box[0] * 8)) +
               C * (2 * (nh + no) * 4 + (nh + ns) * 4 + no * 24) + N * 8 + NH * 8 + (double)C * 9 * 2048 * 8;
   if (o.store_samples) cs += (double)std::max(o.nsave, 1) * (no * 4 + 24) * C;
@@ -3131,14 +3200,14 @@ extern "C" int dr_log_posterior_noalloc(const dr_volume* v, const float* mu_devi
   DevChains ch{};
   ch.C = 1;
   ch.Cp = 1;
-  ch.CG = 1;
   ch.muD = (float*)(base + NA_MUD);
   ch.rs = (float*)(base + NA_RS);
   ch.gD = (float*)(base + NA_GD);
   ch.part = (double*)(base + NA_PART);
   ch.maxblk = NA_MAXBLK;
-  ch.nb_w = std::max(1, std::min(dv.n_s, NA_MAXBLK));
-  ch.nb_wt = std::max(1, std::min(cdiv_i(dv.n_h, 8), NA_MAXBLK));
+  ch.nb_w = std::min(v->nb_w1, NA_MAXBLK);
+  const int sms = device_tables(v->device).sms;
+  ch.nb_wt = std::min(dv.n_s > 0 ? v->nb_wt1 : std::max(1, cdiv_i(dv.n_h, ROWP_NT)), NA_MAXBLK);
   ch.st = st;
   ChainState h;
   std::memset(&h, 0, sizeof(h));
@@ -3152,8 +3221,8 @@ extern "C" int dr_log_posterior_noalloc(const dr_volume* v, const float* mu_devi
   k_gather_re<<<cdiv_i(dv.n_h, 256), 256, 0, s>>>((const float2*)mu_device, dv.d_flat, dv.n_h, ch.muD, 1, 0, dv.N,
                                                    nullptr);
   CK_LAUNCH();
-  if (dv.n_s > 0) launch_spmv_dc(dv, ch, 1, -1, 0, 0, true, s);
-  launch_spmv_dc(dv, ch, 1, -1, 0, 0, false, s);
+  if (dv.n_s > 0) launch_rows(dv, v->rows_w, ch, sms, -1, 0, 0, true, s);
+  launch_rows(dv, v->rows_wt, ch, sms, -1, 0, 0, false, s);
   // u = IFFT(mu) in the scratch field, then the prior's spectral sum
   CK(cudaMemcpyAsync(field, mu_device, sizeof(float2) * dv.N, cudaMemcpyDeviceToDevice, s));
   fft3d<float2>(field, v->hv.E, +1, v->tw_f, s);

@@ -63,19 +63,26 @@ struct DevVolume {
   const int* o_flat;        // [n_o]
   const float* Yh;          // [n_h]
   const float* Ys;          // [n_s]
-  const int* w_rowptr;      // W: n_s x n_h CSR
-  const int* w_col;
-  const float* w_val;
-  const int* wt_rowptr;     // W^T: n_h x n_s CSR
-  const int* wt_col;
-  const float* wt_val;
 };
+
+// W or W^T in groups of ROWP_R consecutive rows (row_products.cuh).  Group g's entries are [ptr[g], ptr[g + 1]) (at least
+// one); entry k has column base[k / 32] + off[k] and its rows' values val[k].
+struct DevRowGroups {
+  int n_rows, n_cols;
+  int groups;               // 0: no rows
+  long long entries;        // padded to ROWP_PAD
+  int stream;               // the matrix is read from memory on every product: ask L2 for entries ahead
+  const int* ptr;           // [groups + 1]
+  const int* base;          // [entries / 32]
+  const uint16_t* off;      // [entries]
+  const float* val;         // [entries][ROWP_R]
+};
+constexpr int ROWP_R = 4, ROWP_PAD = 64;
 
 // The per-chain device buffers of one chainset.
 struct DevChains {
   int C;                    // chains
   int Cp;                   // pitch of the chain-minor arrays (>= C)
-  int CG;                   // lanes per chain group in the kriging kernels (power of two <= 32)
   float2* U;                // [C][2][NH] half spectrum of Re mu: accepted / proposal halves
   float2* G;                // [C][2][NH] half spectrum of Im mu, the same
   float2* Q;                // [C][NH]    half-spectrum momentum of Re mu (that of Im mu lives in k_momentum's registers)

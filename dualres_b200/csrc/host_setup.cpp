@@ -11,9 +11,11 @@
 // numerically positive definite) where the reference uses FP32
 // colPivHouseholderQr.
 #include "host_setup.h"
+#include "drb.h"
 
 #include <algorithm>
 #include <chrono>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -521,6 +523,108 @@ int kriging_build(const float* hr, int nx, int ny, int nz, const float* Qhr, con
 
 
 // ---------------------------------------------------------------- preparation
+namespace {
+
+// Emits the entries of a range of row groups in order: put(column or -1 for a filler, its rows' values) and group(g) before each
+// group's first entry.  A batch of 32 entries is filled up (fillers count to the group before) when the next column
+// would take its columns' span past 65535, and at the end of the range.
+template <class Put, class Group>
+void merge_groups(const std::vector<int>& rowptr, const int* col, const float* val, int g0, int g1, Put&& put,
+                  Group&& group) {
+  constexpr int R = ROWP_R;
+  const int n_rows = (int)rowptr.size() - 1;
+  int n = 0, lo = 0, hi = 0;  // entries so far, the batch's columns
+  const float zero[R] = {};
+  auto fill = [&] {
+    for (; n % 32 != 0; n++) put(-1, zero);
+  };
+  auto room = [&](int c) {
+    if (n % 32 == 0) {
+      lo = hi = c;
+    } else if (std::max(hi, c) - std::min(lo, c) > 65535) {
+      fill();
+      lo = hi = c;
+    } else {
+      lo = std::min(lo, c);
+      hi = std::max(hi, c);
+    }
+  };
+  for (int g = g0; g < g1; g++) {
+    // each row's next nonzero and its column (none: INT_MAX)
+    int head[R], end[R], cur[R];
+    for (int i = 0; i < R; i++) {
+      const int r = g * R + i;
+      head[i] = r < n_rows ? rowptr[r] : 0;
+      end[i] = r < n_rows ? rowptr[r + 1] : 0;
+      cur[i] = head[i] < end[i] ? col[head[i]] : INT_MAX;
+    }
+    bool any = false;
+    for (;;) {
+      int m = cur[0];
+      for (int i = 1; i < R; i++) m = std::min(m, cur[i]);
+      if (m == INT_MAX) {
+        if (any) break;
+        m = n % 32 == 0 ? 0 : lo;  // a group without columns: one entry of value 0
+      }
+      room(m);
+      if (!any) group(g);
+      any = true;
+      float a[R];
+      for (int i = 0; i < R; i++) {
+        a[i] = 0.f;
+        if (cur[i] != m) continue;
+        a[i] = val[head[i]++];
+        cur[i] = head[i] < end[i] ? col[head[i]] : INT_MAX;
+      }
+      put(m, a);
+      n++;
+    }
+  }
+  fill();
+}
+
+}  // namespace
+
+bool row_groups(const std::vector<int>& rowptr, const int* col, const float* val, RowGroupsHost* out) {
+  constexpr int R = ROWP_R, UNIT = 64;  // groups per parallel unit; a unit starts at a batch
+  const int n_rows = (int)rowptr.size() - 1, G = (n_rows + R - 1) / R, units = (G + UNIT - 1) / UNIT;
+  std::vector<long long> first(units + 1, 0);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int u = 0; u < units; u++) {
+    long long n = 0;
+    merge_groups(rowptr, col, val, u * UNIT, std::min(G, (u + 1) * UNIT), [&](int, const float*) { n++; }, [](int) {});
+    first[u + 1] = n;
+  }
+  for (int u = 0; u < units; u++) first[u + 1] += first[u];
+  if (first[units] > INT_MAX - 4096) return false;
+  const size_t n = (size_t)(first[units] + ROWP_PAD - 1) / ROWP_PAD * ROWP_PAD;
+  out->ptr.assign(G + 1, (int)first[units]);
+  out->base.resize(n / 32);
+  out->off.resize(n);
+  out->val.resize(n * R);
+#pragma omp parallel for schedule(dynamic, 1)
+  for (int u = 0; u < units; u++) {
+    size_t k = (size_t)first[u];
+    int cols[32];
+    auto put = [&](int c, const float* a) {
+      std::copy(a, a + R, out->val.begin() + k * R);
+      cols[k % 32] = c;
+      if (++k % 32 != 0) return;
+      int base = INT_MAX;
+      for (int j : cols)
+        if (j >= 0) base = std::min(base, j);
+      out->base[k / 32 - 1] = base;
+      for (int b = 0; b < 32; b++) out->off[k - 32 + b] = (uint16_t)(cols[b] >= 0 ? cols[b] - base : 0);
+    };
+    merge_groups(rowptr, col, val, u * UNIT, std::min(G, (u + 1) * UNIT), put, [&](int g) { out->ptr[g] = (int)k; });
+  }
+  const size_t end = (size_t)first[units];  // the padding is brought to L2 with the last entries and never used
+  std::fill(out->base.begin() + end / 32, out->base.end(), 0);
+  std::fill(out->off.begin() + end, out->off.end(), (uint16_t)0);
+  std::fill(out->val.begin() + end * R, out->val.end(), 0.f);
+  return true;
+}
+
 void build_transpose(HostVolume* hv) {
   const int n_h = (int)hv->Yh.size(), n_s = (int)hv->Ys.size();
   const size_t nnz = hv->w_col.size();

@@ -104,6 +104,17 @@ int kriging_build(const float* hr, int nx, int ny, int nz, const float* Qhr, con
                   const float* Qsr, const float* theta, float radius, std::vector<int>* rowptr, std::vector<int>* col,
                   std::vector<float>* val, int* n_offsets, std::string* err);
 
+// A CSR matrix in groups of ROWP_R consecutive rows over the union of their columns, as DevRowGroups describes it.
+struct RowGroupsHost {
+  std::vector<int> ptr;  // groups + 1
+  fill_vector<int> base;
+  fill_vector<uint16_t> off;
+  fill_vector<float> val;
+  int groups() const { return (int)ptr.size() - 1; }
+};
+// false when the entries would not be addressable with 32-bit positions.
+bool row_groups(const std::vector<int>& rowptr, const int* col, const float* val, RowGroupsHost* out);
+
 // Host part of a dense-tile plan for the tensor-core kriging products: rows
 // ordered along the Z-order curve of their keys (3 x 10-bit coordinates) and
 // cut into tiles of 128; the sorted union of each tile's columns cut into

@@ -898,255 +898,6 @@ __global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETC
   plane_finish<E, NT>(sm, ch, c, z, first, last, pa, pb, T, bx, by, twE, red);
 }
 
-// ----------------------------------------------------------------- kriging products
-// Chain-minor operands: X[j * Cp + c].  A warp's lanes are CG chain lanes x
-// G = 32 / CG nonzero groups; each lane owns NR chains (c = cc + CG r).
-//
-// Batches of 32 nonzeros whose values and columns a warp loads before using any (csr_batches): 8 for 2-8 chains
-// per warp (four chains on a 256x256x128 embedding: W 263 -> 235 us), 2 for one chain (deeper was slower there:
-// 12.5 against 10.2 us on a 32^3 volume) and for 16, 1 for 32 (their gathers already overlap).
-__host__ __device__ constexpr int csr_prefetch(int CG) { return (CG >= 2 && CG <= 8) ? 8 : (CG == 32 ? 1 : 2); }
-
-// Accumulates sum_k val[k] X[col[k]] over the 32-nonzero batches b0, b0 + bs,
-// ... of [ks, ke): the batch's values and columns are loaded once, coalesced,
-// and broadcast by shuffle, so the X loads of a batch are independent and
-// stay in flight together.
-// n_cols bounds the column indices (checked builds; err receives the failure).
-template <int CG, int NR, int PF>
-__device__ __forceinline__ void csr_batches(const float* __restrict__ val, const int* __restrict__ col, int ks, int ke,
-                                            int b0, int bs, const float* const (&x)[NR], int Cp, int lane,
-                                            float (&acc)[NR], int n_cols, int* err) {
-  constexpr int G = 32 / CG;
-  const int grp = lane / CG;
-  if constexpr (PF == 1) {
-    for (int base = ks + b0 * 32; base < ke; base += bs * 32) {
-      const int n = min(32, ke - base);
-      const float mv = lane < n ? __ldg(val + base + lane) : 0.f;
-      const int mc = lane < n ? __ldg(col + base + lane) : 0;
-#pragma unroll
-      for (int j0 = 0; j0 < 32; j0 += G) {
-        const int j = j0 + grp;
-        const float w = __shfl_sync(0xffffffffu, mv, j);
-        const int cj = __shfl_sync(0xffffffffu, mc, j);
-        const long long cidx = (long long)cj * Cp;
-        if (j < n && in_bounds(cj, n_cols, err)) {
-#pragma unroll
-          for (int r = 0; r < NR; r++) acc[r] = fmaf(w, x[r][cidx], acc[r]);
-        }
-      }
-    }
-  } else {
-    // PF batches of values and columns are loaded before any is used, so that several 256-byte loads per warp
-    // are in flight while the matrix streams from memory; the batches are then consumed in their usual order.
-    for (int base = ks + b0 * 32; base < ke; base += PF * bs * 32) {
-      float mvp[PF];
-      int mcp[PF], np[PF];
-#pragma unroll
-      for (int p = 0; p < PF; p++) {
-        const int bb = base + p * bs * 32;
-        np[p] = max(0, min(32, ke - bb));
-        mvp[p] = lane < np[p] ? __ldg(val + bb + lane) : 0.f;
-        mcp[p] = lane < np[p] ? __ldg(col + bb + lane) : 0;
-      }
-#pragma unroll
-      for (int p = 0; p < PF; p++) {
-        const int n = np[p];
-        if (n == 0) break;
-        const float mv = mvp[p];
-        const int mc = mcp[p];
-#pragma unroll
-        for (int j0 = 0; j0 < 32; j0 += G) {
-          const int j = j0 + grp;
-          const float w = __shfl_sync(0xffffffffu, mv, j);
-          const int cj = __shfl_sync(0xffffffffu, mc, j);
-          const long long cidx = (long long)cj * Cp;
-          if (j < n && in_bounds(cj, n_cols, err)) {
-#pragma unroll
-            for (int r = 0; r < NR; r++) acc[r] = fmaf(w, x[r][cidx], acc[r]);
-          }
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < NR; r++)
-#pragma unroll
-    for (int off = CG; off < 32; off <<= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], off);
-}
-
-// rs = Ys - W mu_D for every chain (MultiResParameters.h:361-363, 505-507),
-// one block per row of W (grid-stride over rows); the 8 warps share the
-// row's 32-nonzero batches and combine their sums in a fixed order.
-template <int CG, int NR>
-__global__ void __launch_bounds__(256, 4) k_spmv_w(DevVolume v, DevChains ch, int step, int sel, int chain_only) {
-  grid_dep_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int C = ch.C, Cp = ch.Cp;
-  const int cc = lane % CG;
-  __shared__ float red[8][CG * NR];
-  const float* x[NR];
-#pragma unroll
-  for (int r = 0; r < NR; r++) {
-    const int c = min(cc + CG * r, C - 1);
-    x[r] = ch.muD + (long long)sel * v.n_h * Cp + c;
-  }
-  // thread t < C owns chain t for the row sums
-  const int t = threadIdx.x;
-  bool tact = false;
-  if (t < C && (chain_only < 0 || t == chain_only)) tact = step < 0 || step <= ch.st[t].L_cur;
-  double sq = 0.0;
-  for (int row = blockIdx.x; row < v.n_s; row += gridDim.x) {
-    float acc[NR];
-#pragma unroll
-    for (int r = 0; r < NR; r++) acc[r] = 0.f;
-    // batches ahead keep the matrix stream in flight (csr_prefetch)
-    csr_batches<CG, NR, csr_prefetch(CG)>(v.w_val, v.w_col, v.w_rowptr[row], v.w_rowptr[row + 1], warp, 8, x, Cp,
-                                          lane, acc, v.n_h, ch.err);
-    if (lane < CG) {
-#pragma unroll
-      for (int r = 0; r < NR; r++) red[warp][lane + CG * r] = acc[r];
-    }
-    __syncthreads();
-    if (tact) {
-      float s = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; w++) s += red[w][t];
-      const float rsv = v.Ys[row] - s;
-      ch.rs[(long long)row * Cp + t] = rsv;
-      sq += (double)rsv * rsv;
-    }
-    __syncthreads();
-  }
-  if (tact) {
-    const int slot = step <= 0 ? SL_RS0 : (step == ch.st[t].L_cur ? SL_RSL : SL_SCRATCH);
-    ch.part[((long long)t * NSLOT + slot) * ch.maxblk + blockIdx.x] = sq;
-  }
-}
-
-// The same product with one warp per row of W (grid-stride over rows by warps), for kriging matrices with many
-// rows per block (large volumes with few chains): no block barrier per row, and every warp keeps 8 batches of its
-// row in flight.  The per-chain squared residuals are summed over the block's warps in a fixed order.
-template <int CG, int NR>
-__global__ void __launch_bounds__(256, 4) k_spmv_w_rows(DevVolume v, DevChains ch, int step, int sel, int chain_only) {
-  grid_dep_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int C = ch.C, Cp = ch.Cp;
-  const int cc = lane % CG;
-  __shared__ double red[8][CG * NR];
-  bool act[NR];
-  double sq[NR];
-  const float* x[NR];
-#pragma unroll
-  for (int r = 0; r < NR; r++) {
-    const int c = cc + CG * r;
-    const int cs = min(c, C - 1);
-    x[r] = ch.muD + (long long)sel * v.n_h * Cp + cs;
-    act[r] = false;
-    sq[r] = 0.0;
-    if (c < C && (chain_only < 0 || c == chain_only)) act[r] = step < 0 || step <= ch.st[c].L_cur;
-  }
-  for (int row = blockIdx.x * 8 + warp; row < v.n_s; row += gridDim.x * 8) {
-    float acc[NR];
-#pragma unroll
-    for (int r = 0; r < NR; r++) acc[r] = 0.f;
-    csr_batches<CG, NR, 8>(v.w_val, v.w_col, v.w_rowptr[row], v.w_rowptr[row + 1], 0, 1, x, Cp, lane, acc, v.n_h,
-                           ch.err);
-    if (lane < CG) {
-      const float ys = v.Ys[row];
-#pragma unroll
-      for (int r = 0; r < NR; r++) {
-        if (!act[r]) continue;
-        const float rsv = ys - acc[r];
-        ch.rs[(long long)row * Cp + cc + CG * r] = rsv;
-        sq[r] += (double)rsv * rsv;
-      }
-    }
-  }
-  if (lane < CG) {
-#pragma unroll
-    for (int r = 0; r < NR; r++) red[warp][lane + CG * r] = sq[r];
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    if (chain_only >= 0 && c != chain_only) continue;
-    const ChainState& st = ch.st[c];
-    if (step >= 0 && step > st.L_cur) continue;
-    double t = 0.0;
-    for (int w = 0; w < 8; w++) t += red[w][c];
-    const int slot = step <= 0 ? SL_RS0 : (step == st.L_cur ? SL_RSL : SL_SCRATCH);
-    ch.part[((long long)c * NSLOT + slot) * ch.maxblk + blockIdx.x] = t;
-  }
-}
-
-// gD = sigma_h^-2 (Yh - mu_D) + sigma_s^-2 W^T rs (MultiResParameters.h:357-364),
-// one warp per data voxel over the transposed CSR (grid-stride), plus the
-// ||Yh - mu_D||^2 partials per block.
-template <int CG, int NR>
-__global__ void __launch_bounds__(256, 4) k_spmv_wt(DevVolume v, DevChains ch, int step, int sel, int chain_only) {
-  grid_dep_wait();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int C = ch.C, Cp = ch.Cp;
-  const int cc = lane % CG;
-  __shared__ double red[8][CG * NR];
-  bool act[NR];
-  double sq[NR];
-  int half[NR];
-  float shv[NR], ssv[NR];
-  const float* x[NR];
-#pragma unroll
-  for (int r = 0; r < NR; r++) {
-    const int c = cc + CG * r;
-    const int cs = min(c, C - 1);
-    x[r] = ch.rs + cs;
-    act[r] = false;
-    sq[r] = 0.0;
-    half[r] = 0;
-    shv[r] = ssv[r] = 0.f;
-    if (c < C && (chain_only < 0 || c == chain_only)) {
-      const ChainState& st = ch.st[c];
-      act[r] = step < 0 || step <= st.L_cur;
-      half[r] = sel;
-      shv[r] = st.sh;
-      ssv[r] = st.ss;
-    }
-  }
-  for (int row = blockIdx.x * 8 + warp; row < v.n_h; row += gridDim.x * 8) {
-    float acc[NR];
-#pragma unroll
-    for (int r = 0; r < NR; r++) acc[r] = 0.f;
-    if (v.n_s > 0)
-      csr_batches<CG, NR, csr_prefetch(CG) < 2 ? 2 : csr_prefetch(CG)>(v.wt_val, v.wt_col, v.wt_rowptr[row],
-                                                                       v.wt_rowptr[row + 1], 0, 1, x, Cp, lane, acc,
-                                                                       v.n_s, ch.err);
-    if (lane < CG) {
-      const float yh = v.Yh[row];
-#pragma unroll
-      for (int r = 0; r < NR; r++) {
-        if (!act[r]) continue;
-        const int c = cc + CG * r;
-        const float m = ch.muD[((long long)half[r] * v.n_h + row) * Cp + c];
-        const float rh = yh - m;
-        ch.gD[(long long)row * Cp + c] = shv[r] * rh + ssv[r] * acc[r];
-        sq[r] += (double)rh * rh;
-      }
-    }
-  }
-  if (lane < CG) {
-#pragma unroll
-    for (int r = 0; r < NR; r++) red[warp][lane + CG * r] = sq[r];
-  }
-  __syncthreads();
-  for (int c = threadIdx.x; c < C; c += blockDim.x) {
-    if (chain_only >= 0 && c != chain_only) continue;
-    const ChainState& st = ch.st[c];
-    if (step >= 0 && step > st.L_cur) continue;
-    double s = 0.0;
-    for (int w = 0; w < 8; w++) s += red[w][c];
-    const int slot = step <= 0 ? SL_RH0 : (step == st.L_cur ? SL_RHL : SL_SCRATCH);
-    ch.part[((long long)c * NSLOT + slot) * ch.maxblk + blockIdx.x] = s;
-  }
-}
-
 // ----------------------------------------------------------------- per-iteration scalars
 // The arguments of MultiResParameters::update: eps() and integrator_steps()
 // (gaussian_process_model.h:135).

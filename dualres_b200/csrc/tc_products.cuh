@@ -35,7 +35,7 @@
 //
 // k_tc_finish: one block per 16 rows of a tile sums the tile's segment
 // partials in segment order (deterministic), then applies the epilogue as the
-// CSR kernels k_spmv_w / k_spmv_wt do: rs = Ys - W mu_D with the ||rs||^2
+// row-group kernels do: rs = Ys - W mu_D with the ||rs||^2
 // partials, or gD = sigma_h^-2 (Yh - mu_D) + sigma_s^-2 W^T rs with the
 // ||Yh - mu_D||^2 partials (MultiResParameters.h:357-364).
 #pragma once
