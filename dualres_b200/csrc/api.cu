@@ -1077,8 +1077,6 @@ static void enqueue_steps(Chainset* S, int L, int flags) {
 
 static void enqueue_iteration(Chainset* S) {
   const DevVolume& v = S->vol->dv;
-  k_iter_begin<<<cdiv_i(S->C, 128), 128, 0, S->stream>>>(S->dc);
-  CK_LAUNCH();
   enqueue_steps(S, S->opts.leapfrog, 0);
   k_accept<<<S->C, 256, 0, S->stream>>>(v, S->dc);
   CK_LAUNCH();

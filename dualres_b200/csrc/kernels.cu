@@ -370,12 +370,24 @@ __global__ void __launch_bounds__(MOM_NT) k_momentum(DevVolume v, DevChains ch) 
   __shared__ float2 wa[FIXED ? 1 : MOM_ITEMS], wb[FIXED ? 1 : MOM_ITEMS];
   __shared__ double red[MOM_NT / 32];
   const int c = blockIdx.y;
-  const ChainState& st = ch.st[c];
-  const int L = st.L_cur;
+  ChainState& st = ch.st[c];
+  int L = st.L_cur;
+  float eps = st.eps_cur;
+  if constexpr (!FIXED) {
+    // the arguments of MultiResParameters::update: eps() and integrator_steps() (gaussian_process_model.h:135); every
+    // thread forms them, the first leaves them for the kernels that follow
+    const u32x4 r = philox(u32x4{0u, (uint32_t)st.iteration, (uint32_t)(ch.chain0 + c), RNG_SCALAR}, ch.seed);
+    eps = hmc_eps(st, u01d(r.x, r.y));
+    L = st.done ? -1 : hmc_steps(st);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      if (L >= 0) st.eps_cur = eps;
+      st.L_cur = L;
+    }
+  }
   if (L < 0) return;
   const int E0 = v.E0, E1 = v.E1, E2 = v.E2, acc = st.acc;
   const long long NH = v.NH;
-  const float eps = st.eps_cur, sh = st.sh, Nf = (float)v.N;
+  const float sh = st.sh, Nf = (float)v.N;
   const float2* Gs = ch.G + ((long long)c * 2 + acc) * NH;
   float2* Gd = ch.G + ((long long)c * 2 + (acc ^ 1)) * NH;
   float2* Qc = ch.Q + (long long)c * NH;
@@ -899,46 +911,29 @@ __global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETC
 }
 
 // ----------------------------------------------------------------- per-iteration scalars
-// The arguments of MultiResParameters::update: eps() and integrator_steps()
-// (gaussian_process_model.h:135).
-__global__ void k_iter_begin(DevChains ch) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ch.C) return;
-  ChainState& st = ch.st[c];
-  if (st.done) {
-    st.L_cur = -1;
-    return;
-  }
-  const u32x4 r = philox(u32x4{0u, (uint32_t)st.iteration, (uint32_t)(ch.chain0 + c), RNG_SCALAR}, ch.seed);
-  st.eps_cur = hmc_eps(st, u01d(r.x, r.y));
-  st.L_cur = hmc_steps(st);
-}
-
-__device__ double slot_sum(const DevChains& ch, int c, int slot, int nb, double* red) {
-  double s = 0.0;
-  const double* p = ch.part + ((long long)c * NSLOT + slot) * ch.maxblk;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) s += p[i];
-  return block_sum(s, red);
-}
-
 // Metropolis accept (MultiResParameters.h:702-726), Gibbs sigma draws
 // (:821-838) and HMCParameters::update (HMCParameters.h:259-297).  The
-// Hamiltonian difference is formed in FP64.
+// Hamiltonian difference is formed in FP64.  One block per chain: each warp sums
+// one of the eight partial-sum slots, and two threads draw the two sigmas side by
+// side (12.6 us for one chain with block-wide sums in turn and the draws one after the other).
 __global__ void __launch_bounds__(256) k_accept(DevVolume v, DevChains ch) {
-  __shared__ double red[8];
   __shared__ double sums[8];
-  const int c = blockIdx.x;
+  __shared__ float s_ss;
+  __shared__ int s_err;
+  const int c = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   ChainState& st = ch.st[c];
   if (st.L_cur < 0) return;
-  const int ne = ch.nb_x + ch.nb_g;
-  const int nbs[8] = {ne, ne, ch.nb_wt, ch.nb_w, ne, ne, ch.nb_wt, ch.nb_w};
-  for (int s = 0; s < 8; s++) {
+  {
+    const bool residual_s = warp == SL_RS0 || warp == SL_RSL, residual_h = warp == SL_RH0 || warp == SL_RHL;
+    const int nb = residual_s ? (v.n_s > 0 ? ch.nb_w : 0) : (residual_h ? ch.nb_wt : ch.nb_x + ch.nb_g);
+    const double* p = ch.part + ((long long)c * NSLOT + warp) * ch.maxblk;
     double t = 0.0;
-    if (!((s == SL_RS0 || s == SL_RSL) && v.n_s == 0)) t = slot_sum(ch, c, s, nbs[s], red);
-    if (threadIdx.x == 0) sums[s] = t;
-    __syncthreads();
+#pragma unroll 4
+    for (int i = lane; i < nb; i += 32) t += p[i];
+    t = warp_sum(t);
+    if (lane == 0) sums[warp] = t;
   }
-  if (threadIdx.x != 0) return;
+  __syncthreads();
   const double N = (double)v.N;
   const double sh = st.sh, ss = st.ss;
   const double lp0 = -0.5 * sums[SL_LP0] / N;
@@ -952,24 +947,34 @@ __global__ void __launch_bounds__(256) k_accept(DevVolume v, DevChains ch) {
   if (isnan(R)) R = 0.0;
   const u32x4 r = philox(u32x4{0u, (uint32_t)st.iteration, (uint32_t)(ch.chain0 + c), RNG_SCALAR}, ch.seed);
   const double u = u01d(r.z, r.w);
-  double Rh = sums[SL_RH0], Rs = sums[SL_RS0];
-  ch.moved[c] = u < R;
-  if (u < R) {
+  const bool moved = u < R;
+  const double Rh = moved ? sums[SL_RHL] : sums[SL_RH0], Rs = moved ? sums[SL_RSL] : sums[SL_RS0];
+  // Gibbs: shape n/2 + 1, rate ||residual||^2 / 2 (float arithmetic as in the reference); the first warp draws
+  // sigma_h, the second sigma_s
+  int err = 0;
+  const int n = warp == 0 ? v.n_h : v.n_s;
+  float draw = (float)ss;
+  if (lane == 0 && (warp == 0 || (warp == 1 && n > 0))) {
+    const float shape = 0.5f * (float)n + 1.0f, rate = 0.5f * (float)(warp == 0 ? Rh : Rs);
+    draw = (float)gamma_draw(shape, 1.0 / (double)rate, ch.seed, RNG_SCALAR, ch.chain0 + c, st.iteration,
+                             warp == 0 ? 16u : 4096u, &err);
+  }
+  if (lane == 0 && warp == 1) {
+    s_ss = draw;
+    s_err = err;
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  ch.moved[c] = moved;
+  if (moved) {
     st.acc ^= 1;
     st.accepted += 1;
-    Rh = sums[SL_RHL];
-    Rs = sums[SL_RSL];
   }
   st.Rh_acc = Rh;
   st.Rs_acc = Rs;
-  // Gibbs: shape n/2 + 1, rate ||residual||^2 / 2 (float arithmetic as in the reference)
-  const float shape_h = 0.5f * (float)v.n_h + 1.0f, rate_h = 0.5f * (float)Rh;
-  st.sh = (float)gamma_draw(shape_h, 1.0 / (double)rate_h, ch.seed, RNG_SCALAR, ch.chain0 + c, st.iteration, 16u, &st.err);
-  if (v.n_s > 0) {
-    const float shape_s = 0.5f * (float)v.n_s + 1.0f, rate_s = 0.5f * (float)Rs;
-    st.ss = (float)gamma_draw(shape_s, 1.0 / (double)rate_s, ch.seed, RNG_SCALAR, ch.chain0 + c, st.iteration, 4096u,
-                              &st.err);
-  }
+  st.err += err + s_err;
+  st.sh = draw;
+  st.ss = s_ss;
   st.grad_evals += st.L_cur + 1;
   st.last_log_ratio = logR;
   st.last_E0 = E0;
