@@ -3,6 +3,7 @@
 // One translation unit holds every kernel (kernels.cu) so that template
 // instantiation and the twiddle tables stay in one module.
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <chrono>
 #include <condition_variable>
@@ -3034,13 +3035,32 @@ int dr_mce_summary(const float* img, int nx, int ny, int nz, const float* qform,
   const int n_off = (int)(P.size() / 3);
   const std::vector<float> d = mce_distances(P, qform);
   std::memcpy(distance, d.data(), sizeof(float) * n_off);
-  device_tables(device);
+  const DeviceTables& dt = device_tables(device);
   CK(cudaSetDevice(device));
   const long long nvox = (long long)nx * ny * nz;
-  const int rows = ny * nz;
-  int n_slabs = std::max(1, std::min(32, rows / 256));
-  const int rows_per_slab = cdiv_i(rows, n_slabs);
-  n_slabs = cdiv_i(rows, rows_per_slab);
+  // tasks: 8 offsets along x from a dx0 = 4 mod 8, in the order of the offsets' first
+  std::vector<MceTask> tasks;
+  {
+    std::map<std::array<int, 3>, int> at;
+    for (int o = 0; o < n_off; o++) {
+      const int dx = P[3 * o], dy = P[3 * o + 1], dz = P[3 * o + 2];
+      const int dx0 = ((dx + 36) / 8) * 8 - 36;  // dx >= -20
+      const auto it = at.try_emplace({dz, dy, dx0}, (int)tasks.size());
+      if (it.second) {
+        MceTask t{dy, dz, dx0, {}};
+        std::fill(t.out, t.out + MCE_LAGS, -1);
+        tasks.push_back(t);
+      }
+      tasks[it.first->second].out[dx - dx0] = o;
+    }
+  }
+  const int n_tasks = (int)tasks.size(), rows = ny * nz;
+  MceRows g{nx, ny, nz, 0, 0};
+  g.pitch = MCE_FRONT + (nx + 3) / 4 * 4 + MCE_BACK;
+  g.bw = (nx + 31) / 32 + 3;
+  // four blocks of the pair kernel are resident on an SM; slabs for two rounds of them
+  const int tb = cdiv_i(n_tasks, MCE_THREADS);
+  const int n_slabs = std::max(1, std::min(rows, cdiv_i(8 * dt.sms, tb)));
   cudaStream_t st = nullptr;
   CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
   std::vector<void*> bufs;
@@ -3053,15 +3073,19 @@ int dr_mce_summary(const float* img, int nx, int ny, int nz, const float* qform,
   };
   try {
     float* d_img = (float*)dalloc(sizeof(float) * nvox);
-    int* d_P = (int*)dalloc(sizeof(int) * P.size());
+    float* d_rows = (float*)dalloc(sizeof(float) * (size_t)(rows + 1) * g.pitch);
+    uint32_t* d_bits = (uint32_t*)dalloc(sizeof(uint32_t) * (size_t)(rows + 1) * g.bw);
+    int* d_any = (int*)dalloc(sizeof(int) * (rows + 1));
+    MceTask* d_tasks = (MceTask*)dalloc(sizeof(MceTask) * n_tasks);
     MceSums* d_part = (MceSums*)dalloc(sizeof(MceSums) * (size_t)n_slabs * n_off);
     float* d_cov = (float*)dalloc(sizeof(float) * n_off);
     int* d_np = (int*)dalloc(sizeof(int) * n_off);
     double* d_sums = sums ? (double*)dalloc(sizeof(double) * 3 * n_off) : nullptr;
     CK(cudaMemcpyAsync(d_img, img, sizeof(float) * nvox, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_P, P.data(), sizeof(int) * P.size(), cudaMemcpyHostToDevice, st));
-    const dim3 grid(n_slabs, cdiv_i(n_off, MCE_OFFSETS_PER_CTA));
-    k_mce_partial<<<grid, MCE_THREADS, 0, st>>>(d_img, nx, ny, nz, d_P, n_off, rows_per_slab, d_part);
+    CK(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(MceTask) * n_tasks, cudaMemcpyHostToDevice, st));
+    k_mce_rows<<<rows + 1, 32, 0, st>>>(d_img, g, d_rows, d_bits, d_any);
+    CK_LAUNCH();
+    k_mce_pairs<<<dim3(n_slabs, tb), MCE_THREADS, 0, st>>>(d_rows, d_bits, d_any, g, d_tasks, n_tasks, n_off, d_part);
     CK_LAUNCH();
     k_mce_finish<<<cdiv_i(n_off, 256), 256, 0, st>>>(d_part, n_slabs, n_off, d_cov, d_np, d_sums);
     CK_LAUNCH();

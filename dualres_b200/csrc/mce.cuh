@@ -3,11 +3,21 @@
 //
 // For every lattice offset p and every pair of voxels (x, x + p) inside the
 // grid whose values are both non-zero and not NaN: the sums of x*y, x and y in
-// double and the pair count.  The image (a few MB) stays in L2; a CTA takes a
-// slab of x-rows and a chunk of offsets, walks the rows of the slab with the
-// threads along x (coalesced loads of both rows of a pair), and reduces each
-// offset's sums over the CTA.  A second kernel adds the slabs in a fixed order,
-// so results do not depend on scheduling.
+// double and the pair count.  That is 25,348 offsets times the image: FP64
+// arithmetic, 3 FMAs per offset and voxel, is what bounds it.
+//
+// A task is 8 offsets that differ in x only (dx0 .. dx0 + 7 at one (dy, dz)); a lane
+// has one task, and a warp walks the x rows of its slab together, four voxels
+// at a time: the four x values (one load for the warp) meet a window of eleven y
+// values that slides along the row in registers, so 96 FMAs take one 16-byte
+// load of each row and eight conversions.  Masked values are zero and masks
+// are factors 0 or 1, so that nothing branches; the counts come from bit rows by
+// popcount.  Rows are padded with zeros (dx0 is a multiple of 4: every load is
+// aligned and none is tested), rows outside the grid are a row of zeros, and x
+// rows without data are skipped.  Slabs interleave the rows, which balances
+// them; a second kernel adds the slabs in order, so results do not depend on
+// scheduling.  Measured on a 76x76x60 image, whole call: 3.8 ms (34.3 ms with one
+// voxel pair per thread at a time, masks tested and rows divided out in the loop).
 #pragma once
 
 #include "common.cuh"
@@ -15,71 +25,113 @@
 namespace drb {
 
 constexpr int MCE_THREADS = 128;
-constexpr int MCE_OFFSETS_PER_CTA = 32;
+constexpr int MCE_LAGS = 8;
+constexpr int MCE_FRONT = 32, MCE_BACK = 40;  // zeros before and after a row: dx0 >= -20, dx0 + 7 <= 27
 
 struct MceSums {
   double sxy, sx, sy;
   int n;
 };
+// 8 offsets (dx0 + l, dy, dz): out[l] is the offset's index, or -1 where it is none of the summary's.
+struct MceTask {
+  int dy, dz, dx0;
+  int out[MCE_LAGS];
+};
+// Geometry of the padded rows: pitch floats a row and bw words of mask bits (bit 32 + i is voxel i); row ny * nz is zero.
+struct MceRows {
+  int nx, ny, nz, pitch, bw;
+};
 
-__device__ __forceinline__ bool mce_nonzero(float v) { return !(isnan(v) || v == 0.0f); }
+__global__ void k_mce_rows(const float* __restrict__ img, MceRows g, float* __restrict__ rows, uint32_t* __restrict__ bits,
+                           int* __restrict__ any) {
+  const int r = blockIdx.x, lane = threadIdx.x;  // one warp per row
+  const bool real = r < g.ny * g.nz;
+  float* row = rows + (long long)r * g.pitch;
+  for (int i = lane; i < g.pitch; i += 32) {
+    const int x = i - MCE_FRONT;
+    float v = real && x >= 0 && x < g.nx ? img[(long long)r * g.nx + x] : 0.f;
+    if (isnan(v)) v = 0.f;
+    row[i] = v;
+  }
+  uint32_t some = 0;
+  for (int q = 0; q < g.bw; q++) {
+    const int x = 32 * (q - 1) + lane;
+    const float v = real && x >= 0 && x < g.nx ? img[(long long)r * g.nx + x] : 0.f;
+    const uint32_t b = __ballot_sync(0xffffffffu, !isnan(v) && v != 0.f);
+    if (lane == 0) bits[(long long)r * g.bw + q] = b;
+    some |= b;
+  }
+  if (lane == 0) any[r] = some != 0;
+}
 
-__global__ void __launch_bounds__(MCE_THREADS) k_mce_partial(const float* __restrict__ img, int nx, int ny, int nz,
-                                                            const int* __restrict__ P, int n_off, int rows_per_slab,
-                                                            MceSums* __restrict__ part) {
-  __shared__ double red[3][MCE_THREADS / 32];
-  __shared__ int redn[MCE_THREADS / 32];
-  const int slab = blockIdx.x;
-  const int rows = ny * nz;
-  const int r0 = slab * rows_per_slab, r1 = min(rows, r0 + rows_per_slab);
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int o0 = blockIdx.y * MCE_OFFSETS_PER_CTA, o1 = min(n_off, o0 + MCE_OFFSETS_PER_CTA);
-  for (int o = o0; o < o1; o++) {
-    const int dx = P[3 * o], dy = P[3 * o + 1], dz = P[3 * o + 2];
-    const int i0 = max(0, -dx), i1 = min(nx, nx - dx);
-    double sxy = 0.0, sx = 0.0, sy = 0.0;
-    int n = 0;
-    for (int r = r0; r < r1; r++) {
-      const int j = r % ny, k = r / ny;
-      const int j2 = j + dy, k2 = k + dz;
-      if (j2 < 0 || j2 >= ny || k2 < 0 || k2 >= nz) continue;  // uniform over the CTA
-      const float* xr = img + (long long)r * nx;
-      const float* yr = img + ((long long)k2 * ny + j2) * nx + dx;
-      for (int i = i0 + threadIdx.x; i < i1; i += MCE_THREADS) {
-        const float xv = __ldg(xr + i);
-        if (!mce_nonzero(xv)) continue;
-        const float yv = __ldg(yr + i);
-        if (!mce_nonzero(yv)) continue;
-        sxy += (double)xv * (double)yv;
-        sx += (double)xv;
-        sy += (double)yv;
-        n++;
+__global__ void __launch_bounds__(MCE_THREADS) k_mce_pairs(const float* __restrict__ rows, const uint32_t* __restrict__ bits,
+                                                          const int* __restrict__ any, MceRows g,
+                                                          const MceTask* __restrict__ tasks, int n_tasks, int n_off,
+                                                          MceSums* __restrict__ part) {
+  const int t = blockIdx.y * MCE_THREADS + threadIdx.x;
+  const int nrows = g.ny * g.nz, n4 = (g.nx + 3) / 4, nw = (g.nx + 31) / 32;
+  const MceTask* T = tasks + min(t, n_tasks - 1);
+  const int dy = T->dy, dz = T->dz, dx0 = T->dx0;
+  double sxy[MCE_LAGS], sx[MCE_LAGS], sy[MCE_LAGS];
+  int n[MCE_LAGS];
+#pragma unroll
+  for (int l = 0; l < MCE_LAGS; l++) {
+    sxy[l] = sx[l] = sy[l] = 0.0;
+    n[l] = 0;
+  }
+  for (int r = blockIdx.x; r < nrows; r += gridDim.x) {
+    if (!__ldg(any + r)) continue;  // the same row for the whole block
+    const int j2 = r % g.ny + dy, k2 = r / g.ny + dz;
+    const int r2 = j2 >= 0 && j2 < g.ny && k2 >= 0 && k2 < g.nz ? k2 * g.ny + j2 : nrows;
+    const float4* X = reinterpret_cast<const float4*>(rows + (long long)r * g.pitch + MCE_FRONT);
+    const float4* Y = reinterpret_cast<const float4*>(rows + (long long)r2 * g.pitch + MCE_FRONT + dx0);
+    double w[12], m[12];  // y values and their masks at x .. x + 11 (+ dx0)
+    auto put = [&](int at, float4 v) {
+      const float f[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        w[at + i] = (double)f[i];
+        m[at + i] = f[i] != 0.f ? 1.0 : 0.0;
+      }
+    };
+    put(0, __ldg(Y));
+    put(4, __ldg(Y + 1));
+    for (int i = 0; i < n4; i++) {
+      const float4 xv = __ldg(X + i);
+      put(8, __ldg(Y + i + 2));
+      const float f[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        const double x = (double)f[u], mx = f[u] != 0.f ? 1.0 : 0.0;
+#pragma unroll
+        for (int l = 0; l < MCE_LAGS; l++) {
+          sxy[l] = fma(x, w[u + l], sxy[l]);
+          sx[l] = fma(x, m[u + l], sx[l]);
+          sy[l] = fma(mx, w[u + l], sy[l]);
+        }
+      }
+#pragma unroll
+      for (int l = 0; l < 8; l++) {
+        w[l] = w[l + 4];
+        m[l] = m[l + 4];
       }
     }
-    for (int off = 16; off > 0; off >>= 1) {
-      sxy += __shfl_xor_sync(0xffffffffu, sxy, off);
-      sx += __shfl_xor_sync(0xffffffffu, sx, off);
-      sy += __shfl_xor_sync(0xffffffffu, sy, off);
-      n += __shfl_xor_sync(0xffffffffu, n, off);
-    }
-    if (lane == 0) {
-      red[0][warp] = sxy;
-      red[1][warp] = sx;
-      red[2][warp] = sy;
-      redn[warp] = n;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      MceSums s{0.0, 0.0, 0.0, 0};
-      for (int w = 0; w < MCE_THREADS / 32; w++) {
-        s.sxy += red[0][w];
-        s.sx += red[1][w];
-        s.sy += red[2][w];
-        s.n += redn[w];
+    const uint32_t* bx = bits + (long long)r * g.bw + 1;
+    const uint32_t* by = bits + (long long)r2 * g.bw;
+    for (int q = 0; q < nw; q++) {
+      const uint32_t x = __ldg(bx + q);
+#pragma unroll
+      for (int l = 0; l < MCE_LAGS; l++) {
+        const int p = 32 + 32 * q + dx0 + l;  // >= 12
+        n[l] += __popc(x & __funnelshift_r(__ldg(by + (p >> 5)), __ldg(by + (p >> 5) + 1), p & 31));
       }
-      part[(long long)slab * n_off + o] = s;
     }
-    __syncthreads();
+  }
+  if (t >= n_tasks) return;
+#pragma unroll
+  for (int l = 0; l < MCE_LAGS; l++) {
+    const int o = T->out[l];
+    if (o >= 0) part[(long long)blockIdx.x * n_off + o] = MceSums{sxy[l], sx[l], sy[l], n[l]};
   }
 }
 
