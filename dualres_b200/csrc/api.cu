@@ -137,7 +137,7 @@ struct DeviceTables {
   // pool is left as it is.
   cudaMemPool_t pool = nullptr;
   int sms = 148;
-  int tma_dyn_max = 0;  // dynamic shared memory available to the bulk-copy plane kernel
+  int plane_dyn_max = 0;  // dynamic shared memory available to the plane kernels
   bool tc = false;      // the tensor-core kriging products fit this device's shared memory
   const float2* tw_f = nullptr;
   const double2* tw_d = nullptr;
@@ -178,11 +178,43 @@ static void set_pass_attrs() {
   }
 }
 
-template <int E, bool PF>
-static void set_plane_attr(int dyn_max) {
-  const PlaneLayout Ly = plane_layout(E, PlaneGeom<E>::SIZE, PF);
-  if (Ly.total <= dyn_max)
-    CK(cudaFuncSetAttribute(k_xyplane<E, PF>, cudaFuncAttributeMaxDynamicSharedMemorySize, Ly.total));
+// Bytes of dynamic shared memory of k_xyplane for a box bx columns wide.
+template <int E0, int E1, bool WIDE>
+static int plane_smem(int bx) {
+  return (plane_box_elems<E0, E1>(bx) + PlaneCfg<E0, E1, WIDE>::ROW_ELEMS) * (int)sizeof(float2);
+}
+// Calls f(integral_constant E) for the square planes that k_plane_square takes; false for the others.
+template <class F>
+static bool square_sizes(int E0, int E1, F&& f) {
+  if (E0 != E1) return false;
+  switch (E0) {
+    case 4: f(std::integral_constant<int, 4>()); return true;
+    case 8: f(std::integral_constant<int, 8>()); return true;
+    case 16: f(std::integral_constant<int, 16>()); return true;
+    case 32: f(std::integral_constant<int, 32>()); return true;
+    case 64: f(std::integral_constant<int, 64>()); return true;
+    default: return false;
+  }
+}
+// Calls f(integral_constant E0, integral_constant E1) for the plane sizes of k_xyplane; false for the others.
+template <class F>
+static bool plane_sizes(int E0, int E1, F&& f) {
+  auto with0 = [&](auto e0) {
+    switch (E1) {
+      case 16: f(e0, std::integral_constant<int, 16>()); return true;
+      case 32: f(e0, std::integral_constant<int, 32>()); return true;
+      case 64: f(e0, std::integral_constant<int, 64>()); return true;
+      case 128: f(e0, std::integral_constant<int, 128>()); return true;
+      default: return false;
+    }
+  };
+  switch (E0) {
+    case 16: return with0(std::integral_constant<int, 16>());
+    case 32: return with0(std::integral_constant<int, 32>());
+    case 64: return with0(std::integral_constant<int, 64>());
+    case 128: return with0(std::integral_constant<int, 128>());
+    default: return false;
+  }
 }
 
 template <class C>
@@ -229,13 +261,16 @@ static DeviceTables& device_tables(int dev) {
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     t.sms = sms;
-    t.tma_dyn_max = optin - 256;  // the plane kernels' static shared memory is at most 128 bytes
-    set_plane_attr<4, false>(t.tma_dyn_max); set_plane_attr<8, false>(t.tma_dyn_max);
-    set_plane_attr<16, false>(t.tma_dyn_max); set_plane_attr<32, false>(t.tma_dyn_max);
-    set_plane_attr<64, false>(t.tma_dyn_max); set_plane_attr<128, false>(t.tma_dyn_max);
-    set_plane_attr<4, true>(t.tma_dyn_max); set_plane_attr<8, true>(t.tma_dyn_max);
-    set_plane_attr<16, true>(t.tma_dyn_max); set_plane_attr<32, true>(t.tma_dyn_max);
-    set_plane_attr<64, true>(t.tma_dyn_max);
+    t.plane_dyn_max = optin - 2560;  // the plane kernels' static shared memory (twiddles, sums) is at most 2.2 KB
+    for (int e0 = 16; e0 <= 128; e0 *= 2)
+      for (int e1 = 16; e1 <= 128; e1 *= 2)
+        plane_sizes(e0, e1, [&](auto a, auto b) {
+          // boxes of up to half the embedding and its middle (bx <= E0 / 2 + 2)
+          set_smem(k_xyplane<a.value, b.value, false>, std::min(t.plane_dyn_max, plane_smem<a.value, b.value, false>(a.value / 2 + 2)));
+          set_smem(k_xyplane<a.value, b.value, true>, std::min(t.plane_dyn_max, plane_smem<a.value, b.value, true>(a.value / 2 + 2)));
+        });
+    set_smem(k_plane_square<64, false>, PlaneGeom<64>::SIZE * (int)sizeof(float2));
+    set_smem(k_plane_square<64, true>, PlaneGeom<64>::SIZE * (int)sizeof(float2));
     CK(cudaFuncSetAttribute(k_kriging_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(KrigSmem)));
     int smax = 0;
     for (int n = 16; n <= 256; n *= 2) smax = std::max(smax, tc_smem_bytes(n));
@@ -771,8 +806,8 @@ struct Chainset {
   std::vector<void*> allocs;
   float2* tmp = nullptr;        // [N] scratch for evaluation calls
   int sms = 148;
-  bool plane = false;           // fused xy-plane update (E0 == E1 <= 128)
-  int path = 0;                 // 0 plane kernel, 1 plane kernel with bulk prefetch, 2 x-line kernel + y passes
+  bool plane = false;           // fused xy-plane update (E0, E1 <= 128)
+  int path = 0;                 // 0 plane kernel, 1 k_xyplane on a small square plane, 2 x-line kernel + y passes
   int grid = 8;                 // kriging-product blocks per SM
   double tuned_ms = 0.0;        // iteration time of the chosen configuration when it was tuned (0: not tuned)
   bool tcp = false;             // kriging products on the tensor cores (dense tiles of the volume)
@@ -780,8 +815,8 @@ struct Chainset {
   float* tc_partial = nullptr;  // [segments][tc_N][128] partial products
   bool tc_tg = false;           // the chain vectors arrive by TMA row gathers over tc_map_w / tc_map_wt
   CUtensorMap tc_map_w{}, tc_map_wt{};  // mu_D as [2 n_h] rows; rs as [n_s] rows
-  bool tma = false;             // path 1
-  int tma_smem = 0, tma_grid = 0;
+  bool wide = false;            // wide blocks of the plane kernels
+  bool rows_plane = false;      // path 1: k_xyplane where k_plane_square is the plane kernel
 
   int64_t bytes = 0;
   cudaEvent_t done_event = nullptr;  // recorded after the last launched iteration (server)
@@ -993,38 +1028,26 @@ static void launch_xline(Chainset* S, int step, int flags) {
   CK_LAUNCH();
 }
 
-template <int E, bool PF>
-static void launch_plane_t(Chainset* S, int step, int flags) {
+static void launch_plane(Chainset* S, int step, int flags) {
   flags |= l2_prefetch_flag();
   const DevVolume& v = S->vol->dv;
-  const dim3 grid(v.EZ, S->C);
-  const size_t smem = (size_t)plane_layout(E, PlaneGeom<E>::SIZE, PF).total;
-  launch_k(k_xyplane<E, PF>, grid, PlaneCfg<E, PF>::NT, smem, S->stream, v, S->dc, step, flags, S->vol->tw_f);
-  CK_LAUNCH();
-}
-
-static void launch_plane(Chainset* S, int step, int flags) {
-  const DevVolume& v = S->vol->dv;
   if (v.EZ > S->dc.maxblk) throw Error(DR_ERR_STATE, "partial-sum buffer smaller than the plane count");
-  if (S->tma) {
-    switch (v.E0) {
-      case 4: launch_plane_t<4, true>(S, step, flags); return;
-      case 8: launch_plane_t<8, true>(S, step, flags); return;
-      case 16: launch_plane_t<16, true>(S, step, flags); return;
-      case 32: launch_plane_t<32, true>(S, step, flags); return;
-      case 64: launch_plane_t<64, true>(S, step, flags); return;
-      default: throw Error(DR_ERR_UNSUPPORTED, "plane size not supported by the bulk-copy kernel");
-    }
-  }
-  switch (v.E0) {
-    case 4: launch_plane_t<4, false>(S, step, flags); break;
-    case 8: launch_plane_t<8, false>(S, step, flags); break;
-    case 16: launch_plane_t<16, false>(S, step, flags); break;
-    case 32: launch_plane_t<32, false>(S, step, flags); break;
-    case 64: launch_plane_t<64, false>(S, step, flags); break;
-    case 128: launch_plane_t<128, false>(S, step, flags); break;
-    default: throw Error(DR_ERR_UNSUPPORTED, "plane size not supported");
-  }
+  const dim3 grid(v.EZ, S->C);
+  auto go = [&](auto wide) {
+    constexpr bool W = decltype(wide)::value;
+    return (!S->rows_plane && square_sizes(v.E0, v.E1, [&](auto a) {
+              launch_k(k_plane_square<a.value, W>, grid, SquareCfg<W>::NT, PlaneGeom<a.value>::SIZE * sizeof(float2), S->stream,
+                       v, S->dc, step, flags, S->vol->tw_f);
+            })) ||
+           plane_sizes(v.E0, v.E1, [&](auto a, auto b) {
+             launch_k(k_xyplane<a.value, b.value, W>, grid, PlaneCfg<a.value, b.value, W>::NT,
+                      plane_smem<a.value, b.value, W>(v.bx), S->stream, v, S->dc, step, flags, S->vol->tw_f);
+           });
+  };
+  // wide blocks while every plane has an SM of its own (and their shared memory fits)
+  const bool ok = S->wide ? go(std::true_type()) : go(std::false_type());
+  if (!ok) throw Error(DR_ERR_UNSUPPORTED, "plane size not supported");
+  CK_LAUNCH();
 }
 
 // The momentum of an iteration and the trajectory of Im mu (k_momentum); with XF_FIXED_MOMENTUM from Gq.
@@ -1258,22 +1281,29 @@ static bool tc_env_off() {
   return e && std::string(e) == "0";
 }
 
+// The plane kernels of a volume: any (plane), k_xyplane besides k_plane_square (alternative), and whether an untuned chain
+// set takes the plane path (square planes).
 struct PathOptions {
-  bool plane = false, prefetch = false;
+  bool plane = false, alternative = false, by_default = false, wide = true;
 };
 static PathOptions path_options(const DevVolume& v, int device) {
   PathOptions po;
-  if (!(v.E0 == v.E1 && v.E0 >= 4 && v.E0 <= 128)) return po;
-  const DeviceTables& dt = device_tables(device);
-  const int elems = v.E0 == 64 ? PlaneGeom<64>::SIZE : (v.E0 == 128 ? PlaneGeom<128>::SIZE : v.E0 * (v.E0 + 1));
-  po.plane = plane_layout(v.E0, elems, false).total <= dt.tma_dyn_max;
-  po.prefetch = po.plane && v.E0 <= 64 && plane_layout(v.E0, elems, true).total <= dt.tma_dyn_max;
+  const int dyn_max = device_tables(device).plane_dyn_max;
+  bool rows = false;
+  plane_sizes(v.E0, v.E1, [&](auto a, auto b) { 
+    rows = v.bx <= v.E0 / 2 + 2 && plane_smem<a.value, b.value, false>(v.bx) <= dyn_max;
+    po.wide = plane_smem<a.value, b.value, true>(v.bx) <= dyn_max;
+  });
+  const bool square = square_sizes(v.E0, v.E1, [](auto) {});
+  po.plane = rows || square;
+  po.alternative = rows && square;
+  po.by_default = po.plane && v.E0 == v.E1;
   return po;
 }
 
 struct TuneChoice {
   int ztile = 8;     // chains per z-pass tile (8 or 1) for chain sets of 8 or more chains
-  int path = 0;      // 0 plane, 1 plane + prefetch, 2 x-line
+  int path = 0;      // 0 plane, 1 k_xyplane on a small square plane, 2 x-line
   int grid = 8;      // kriging-product blocks per SM (row-group products)
   double ms = 0.0;   // measured milliseconds per iteration
   int tc = 0;        // 1: kriging products on the tensor cores
@@ -1371,7 +1401,7 @@ static TuneChoice autotune(Volume* V, int C, const dr_hmc_opts* o) {
     }
   };
   for (int path : {0, 1, 2}) {
-    if ((path == 0 && !po.plane) || (path == 1 && !po.prefetch)) continue;
+    if ((path == 0 && !po.plane) || (path == 1 && !po.alternative)) continue;
     try_candidate(TuneChoice{8, path, 8, 0.0, tc ? 1 : 0});
   }
   if (best.ms < 1e300) {
@@ -1397,7 +1427,7 @@ static TuneChoice autotune(Volume* V, int C, const dr_hmc_opts* o) {
   }
   if (!(best.ms < 1e300)) {  // nothing could be timed: default, not cached
     TuneChoice d;
-    d.path = po.plane ? 0 : 2;
+    d.path = po.by_default ? 0 : 2;
     return d;
   }
   std::lock_guard<std::mutex> lk(g_tune_mtx);
@@ -1431,7 +1461,7 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   S->sms = device_tables(V->device).sms;
   const long long N = v.N, NH = v.NH;
   const PathOptions po = path_options(v, V->device);
-  int path = po.plane ? 0 : 2, grid = 8;
+  int path = po.by_default ? 0 : 2, grid = 8;
   // tensor-core products by default for 32 or more chains; the tuner, DRB_TC_PRODUCTS=0 / 1 and a forced choice
   // override the default
   int tc = C >= 32 ? 1 : 0;
@@ -1449,7 +1479,7 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   } else if (std::getenv("DRB_NO_PLANE")) {
     path = 2;
   } else if (std::getenv("DRB_PLANE_PREFETCH")) {
-    path = po.prefetch ? 1 : path;
+    path = po.alternative ? 1 : (po.plane ? 0 : path);  // k_xyplane wherever it exists
   } else if (autotune_enabled()) {
     const TuneChoice t = autotune(V, C, o);
     path = t.path;
@@ -1462,7 +1492,7 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   if (!forced) {
     if (const char* g = std::getenv("DRB_PRODUCT_BLOCKS_PER_SM")) grid = std::max(1, std::min(16, std::atoi(g)));
   }
-  if ((path == 0 && !po.plane) || (path == 1 && !po.prefetch)) path = po.plane ? 0 : 2;
+  if ((path == 0 && !po.plane) || (path == 1 && !po.alternative)) path = po.by_default ? 0 : 2;
   // the state arrays are allocated after the tuning, whose candidate chain sets then reuse the pool's memory
   // without this chain set's arrays held beside them
   ch.U = S->alloc<float2>((size_t)C * 2 * NH);
@@ -1472,7 +1502,8 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
   S->path = path;
   S->grid = grid;
   S->plane = path != 2;
-  S->tma = path == 1;
+  S->rows_plane = path == 1;
+  S->wide = po.wide && (long long)v.EZ * C <= S->sms;
   ch.t2_stride = (long long)v.EZ * v.by * v.bx;
   if (S->plane) {
     // T1 is only needed by the initial transforms: borrow the momentum buffer

@@ -17,6 +17,8 @@
 // reference).
 #pragma once
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace drb {
@@ -256,7 +258,7 @@ __host__ __device__ constexpr int tw_offset(int N) { return N - 2; }
 constexpr int TW_TOTAL = 1022;
 
 // ----------------------------------------------------------------- padded 2D planes
-// An E x E plane stored with one pad slot after every 8 elements along both
+// An E x E plane (k_plane_square) stored with one pad slot after every 8 elements along both
 // axes: phys(y, x) = (y + y/8) * RP + x + x/8, with the row pitch RP = 8 mod 16
 // (complex units).  With the lane mappings below, every shared-memory access
 // of the two radix stages (including the stride-8 transpose between them) hits
@@ -341,7 +343,7 @@ __device__ __forceinline__ void plane_stage(float2* sm, At at, const int (&bl)[P
 // Row FFTs (lines = y rows, elements along x) of a padded plane, all E rows; x >= rlim read as zero, x >= wlim not
 // written.
 template <int E, int R1, int R2, int DIR>
-__device__ __forceinline__ void plane_rows(float2* sm, const float2* __restrict__ tw, int rlim = E, int wlim = E) {
+__device__ __forceinline__ void plane_rows_padded(float2* sm, const float2* __restrict__ tw, int rlim = E, int wlim = E) {
   using PL = PaddedPlane<E>;
   constexpr int NBM = Plan2<E, R1, R2>::NBM, LPW = 32 / NBM;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -361,7 +363,7 @@ __device__ __forceinline__ void plane_rows(float2* sm, const float2* __restrict_
 // Column FFTs (lines = x columns, elements along y) of the first ncols columns; y >= rlim read as zero, y >= wlim
 // not written.
 template <int E, int R1, int R2, int DIR>
-__device__ __forceinline__ void plane_cols(float2* sm, int ncols, const float2* __restrict__ tw, int rlim = E,
+__device__ __forceinline__ void plane_cols_padded(float2* sm, int ncols, const float2* __restrict__ tw, int rlim = E,
                                            int wlim = E) {
   using PL = PaddedPlane<E>;
   constexpr int NBM = Plan2<E, R1, R2>::NBM, PL_LANE = NBM / 4;
@@ -400,6 +402,160 @@ __device__ __forceinline__ void plane_cols(float2* sm, int ncols, const float2* 
     plane_stage<E, R2, R1, DIR, PL_LANE>(sm, at, bl, on, tw, E, wlim);
   }
   __syncthreads();
+}
+
+// ----------------------------------------------------------------- planes, pruned to a box
+// Column transforms (elements along y) of the first ncols columns of an array of rows of the given pitch (complex), in
+// place; y >= rlim read as zero (never loaded), y >= wlim not written.  A warp's lanes are 16 columns x 2 butterflies, so
+// that a half-warp always touches 16 adjacent points; W warps share a group of 16 columns and synchronise their two
+// stages on a named barrier of their own.
+__device__ __forceinline__ void cols_sync(int bar, int threads) {
+  if (threads == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(threads) : "memory");
+}
+template <int N, int R, int P, int DIR, int NB_LANE>
+__device__ __forceinline__ void col_stage(float2* col, int pitch, bool on, int b0, int bstep, const float2* __restrict__ tw,
+                                          int rlim, int wlim, int bar, int threads) {
+  constexpr int M = N / P, Mn = M / R, NB = N / R;
+  float2 x[NB_LANE][R];
+#pragma unroll
+  for (int q = 0; q < NB_LANE; q++) {
+    const int b = b0 + bstep * q;
+    if (on && b < NB) {
+      const int p = b / Mn, t = b % Mn, i0 = p * M + t;
+#pragma unroll
+      for (int j = 0; j < R; j++) x[q][j] = i0 + Mn * j < rlim ? col[(i0 + Mn * j) * pitch] : make_float2(0.f, 0.f);
+      reg_fft<R, DIR>(x[q]);
+      if (Mn > 1) {
+#pragma unroll
+        for (int k = 1; k < R; k++) {
+          float2 wv = tw[P * t * k];
+          if (DIR > 0) wv.y = -wv.y;
+          x[q][k] = cmul(x[q][k], wv);
+        }
+      }
+    }
+  }
+  cols_sync(bar, threads);
+#pragma unroll
+  for (int q = 0; q < NB_LANE; q++) {
+    const int b = b0 + bstep * q;
+    if (on && b < NB) {
+      const int p = b / Mn, t = b % Mn, o0 = p * Mn + t;
+#pragma unroll
+      for (int k = 0; k < R; k++)
+        if (o0 + P * Mn * k < wlim) col[(o0 + P * Mn * k) * pitch] = x[q][k];
+    }
+  }
+  cols_sync(bar, threads);
+}
+template <int N> struct ColPlan {
+  static constexpr int R1 = N == 128 ? 16 : (N >= 32 ? 8 : 4), R2 = N / R1;
+  static constexpr int NB1 = N / R1, NB2 = N / R2;
+};
+template <int N, int DIR, int W>
+__device__ __forceinline__ void plane_cols_w(float2* sm, int pitch, int ncols, const float2* __restrict__ tw, int rlim, int wlim) {
+  using PL = ColPlan<N>;
+  constexpr int L1 = cdiv(PL::NB1, 2 * W), L2 = cdiv(PL::NB2, 2 * W);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int slot = warp / W, b0 = 2 * (warp % W) + (lane >> 4);
+#pragma unroll 1
+  for (int base = slot * 16; base < ncols; base += nw / W * 16) {
+    const int x = base + (lane & 15);
+    const bool on = x < ncols;
+    float2* col = sm + (on ? x : 0);
+    col_stage<N, PL::R1, 1, DIR, L1>(col, pitch, on, b0, 2 * W, tw, rlim, N, 1 + slot, 32 * W);
+    col_stage<N, PL::R2, PL::R1, DIR, L2>(col, pitch, on, b0, 2 * W, tw, N, wlim, 1 + slot, 32 * W);
+  }
+}
+// For blocks of 8 warps: 4 warps to a group for transforms of 128 (a lane then holds at most 32 points) and while there
+// are at most two groups, else 2.
+template <int N, int DIR>
+__device__ __forceinline__ void plane_cols(float2* sm, int pitch, int ncols, const float2* __restrict__ tw, int rlim, int wlim) {
+  if (N == 128 || ncols <= 32) plane_cols_w<N, DIR, 4>(sm, pitch, ncols, tw, rlim, wlim);
+  else plane_cols_w<N, DIR, N == 128 ? 4 : 2>(sm, pitch, ncols, tw, rlim, wlim);
+}
+
+// Row transforms with the middle in registers.  N = RA x RB, LN = N / RA lanes per
+// row (lane = b + LN row of the warp's ROWS rows), each with RA points:
+//   inverse: radix RA on points b + RB j, exchange, radix RB;
+//   the lane then holds points p + RA k (k < RB) of NBF = RA / LN butterflies
+//   p = 2 b + (m & 1) + 2 LN (m >> 1): pairs of adjacent points, 16-byte loads and
+//   stores of the state in runs of 16 LN bytes;
+//   forward: radix RB on the same points, exchange, radix RA, points b + RB k out.
+// One exchange per direction, through a buffer of the row (point i at pos(i), row
+// pitch RP): a warp's four passes over it take 160 (N = 128) and 192 (N = 64)
+// wavefronts, 128 without any bank conflict; the other paddings take more.
+template <int N> struct RowPlan {
+  static constexpr int RA = N >= 64 ? 16 : 8, RB = N / RA, LN = N / RA, ROWS = 32 / LN, NBF = RA / LN;
+  static constexpr int RP = N == 128 ? 136 : (N == 64 ? 68 : (N == 32 ? 36 : 18));
+  __host__ __device__ static constexpr int pos(int i) { return N >= 64 ? i + (i >> 4) : i + (i >> 3); }
+  __device__ static int butterfly(int b, int m) { return 2 * b + (m & 1) + 2 * LN * (m >> 1); }
+};
+// Pitch (complex) of an array of rows of n points that row transforms of length N read and write: half-warps touch LN
+// adjacent points of 16 / LN rows, which this pitch spreads over the banks.
+template <int N>
+__host__ __device__ constexpr int row_pitch(int n) {
+  const int c = N == 128 ? 8 : (N == 16 ? 2 : 4);
+  return n <= c ? c : (n - c + 15) / 16 * 16 + c;
+}
+
+// Points x < n of a row (in) through the inverse transform into e[m][k] (point p(m) + RA k).
+template <int N>
+__device__ __forceinline__ void row_inverse(const float2* in, int n, float2* row, int b, const float2* __restrict__ tw,
+                                            float2 (&e)[RowPlan<N>::NBF][RowPlan<N>::RB]) {
+  using PL = RowPlan<N>;
+  constexpr int RA = PL::RA, RB = PL::RB;
+  float2 a[RA];
+#pragma unroll
+  for (int j = 0; j < RA; j++) a[j] = b + RB * j < n ? in[b + RB * j] : make_float2(0.f, 0.f);
+  reg_fft<RA, +1>(a);
+#pragma unroll
+  for (int k = 1; k < RA; k++) {
+    float2 w = tw[b * k];
+    w.y = -w.y;
+    a[k] = cmul(a[k], w);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int k = 0; k < RA; k++) row[PL::pos(k * RB + b)] = a[k];
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < PL::NBF; m++) {
+    const float2* s = row + PL::pos(RB * PL::butterfly(b, m));  // RB points that no padding parts
+#pragma unroll
+    for (int j = 0; j < RB; j++) e[m][j] = s[j];
+  }
+#pragma unroll
+  for (int m = 0; m < PL::NBF; m++) reg_fft<RB, +1>(e[m]);
+}
+// e[m][k] through the forward transform to points x < n of a row (out).
+template <int N>
+__device__ __forceinline__ void row_forward(float2 (&e)[RowPlan<N>::NBF][RowPlan<N>::RB], float2* row, int b,
+                                            const float2* __restrict__ tw, float2* out, int n) {
+  using PL = RowPlan<N>;
+  constexpr int RA = PL::RA, RB = PL::RB;
+#pragma unroll
+  for (int m = 0; m < PL::NBF; m++) {
+    reg_fft<RB, -1>(e[m]);
+    const int p = PL::butterfly(b, m);
+#pragma unroll
+    for (int k = 1; k < RB; k++) e[m][k] = cmul(e[m][k], tw[p * k]);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < PL::NBF; m++)
+#pragma unroll
+    for (int k = 0; k < RB; k++) row[PL::pos(k * RA + PL::butterfly(b, m))] = e[m][k];
+  __syncwarp();
+  float2 a[RA];
+  const float2* s = row + PL::pos(b * RA);
+#pragma unroll
+  for (int j = 0; j < RA; j++) a[j] = s[PL::pos(j)];  // b RA is a multiple of the padding's period
+  reg_fft<RA, -1>(a);
+#pragma unroll
+  for (int k = 0; k < RA; k++)
+    if (b + RB * k < n) out[b + RB * k] = a[k];
 }
 
 }  // namespace drb

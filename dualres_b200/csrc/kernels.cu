@@ -624,22 +624,18 @@ __global__ void __launch_bounds__(XCfg<E0>::NT, XCfg<E0>::MINB) k_xline(DevVolum
   }
 }
 
-// ----------------------------------------------------------------- xy-plane kernel
+// ----------------------------------------------------------------- square plane kernel
 // The leapfrog update fused with the y and x transforms of one z-plane of one
 // chain (E0 == E1 == E), one block per (z-plane, chain):
 //   T2[c][z][y < by][x < bx] --inverse y (columns x < bx), inverse x (rows)-->
 //   spectral plane; kick / drift as in k_xline; forward x, forward y --> T2.
-// For E = 64 and 128 the plane uses the padded layout of PaddedPlane (bank-
-// conflict free radix stages); other sizes use an odd row pitch.  With
-// PREFETCH the plane's U and q planes are brought into shared memory at
-// entry by bulk asynchronous copies (1D TMA, completion on an mbarrier) so
-// that their DRAM latency overlaps the inverse transforms; 1/lambda, one array
-// shared by every chain, stays in L2.  The wait is bounded and a time-out is
-// recorded in ch.err.
+// For E = 64 the plane uses the padded layout of PaddedPlane (bank-conflict free
+// radix stages); smaller planes an odd row pitch.  Square planes up to 64 only: the
+// whole plane is in shared memory, four blocks to an SM at E = 64.
 template <int E>
 struct PlaneGeom {
-  static constexpr bool PADDED = (E == 64 || E == 128);
-  static constexpr int R1 = E == 128 ? 16 : 8, R2 = 8;
+  static constexpr bool PADDED = E == 64;
+  static constexpr int R1 = 8, R2 = 8;
   static constexpr int P = E + 1;  // odd pitch of the unpadded layout
   static constexpr int SIZE = PADDED ? PaddedPlane<E>::SIZE : E * (E + 1);
   __device__ __forceinline__ static int at(int y, int x) {
@@ -648,28 +644,13 @@ struct PlaneGeom {
   }
 };
 
-// PREFETCH: the U and q planes are bulk-copied into shared memory at entry; 256 threads and 128 registers, two
-// blocks per SM (E <= 64).  Without it a register budget for three blocks of 256 threads (E <= 64): 80 registers
-// and 80 B of spill against 64 registers and 200 B for four, which with the state prefetched into L2 is the faster
-// (64^2 plane x 64 chains 150.0 against 150.9 us, one chain 10.8 against 12.4 us).
-template <int E, bool PREFETCH> struct PlaneCfg {
-  static constexpr int NT = E >= 128 ? 512 : 256;
-  static constexpr int MINB = PREFETCH ? 2 : (E <= 64 ? 3 : 1);  // blocks per SM the register budget targets
+// 256 threads, four blocks per SM at 64 registers for E = 64 (64 chains on a 64^3 embedding: 68.3 us, 72.4 with three
+// blocks at 80 registers, 79.9 with two blocks of 512 threads).
+// WIDE: 512 threads with all the registers, for chain sets of at most a plane per SM (one chain on 64^3: 7.5 us, 9.0 with
+// the narrow blocks).
+template <bool WIDE> struct SquareCfg {
+  static constexpr int NT = WIDE ? 512 : 256, MINB = WIDE ? 1 : 4;
 };
-
-// Shared-memory layout in bytes: [mbarrier | plane | U | q].
-struct PlaneLayout {
-  int plane_off, u_off, q_off, total;
-};
-__host__ __device__ inline PlaneLayout plane_layout(int E, int plane_elems, bool prefetch) {
-  PlaneLayout L;
-  L.plane_off = prefetch ? 128 : 0;
-  const int pe = (L.plane_off + plane_elems * 8 + 127) / 128 * 128;
-  L.u_off = pe;
-  L.q_off = pe + E * E * 8;
-  L.total = prefetch ? L.q_off + E * E * 8 : L.plane_off + plane_elems * 8;
-  return L;
-}
 
 // The padded planes prune both transforms to the box (ncols x nrows of T2): the inverse transforms read only the
 // box (everything else is zero and is never stored), and the forward transforms write only what lands in it.
@@ -678,11 +659,11 @@ __device__ __forceinline__ void plane_fft(float2* sm, int ncols, int nrows, int 
   using G = PlaneGeom<E>;
   if constexpr (G::PADDED) {
     if (dir > 0) {
-      plane_cols<E, G::R1, G::R2, +1>(sm, ncols, tw, nrows, E);
-      plane_rows<E, G::R1, G::R2, +1>(sm, tw, ncols, E);
+      plane_cols_padded<E, G::R1, G::R2, +1>(sm, ncols, tw, nrows, E);
+      plane_rows_padded<E, G::R1, G::R2, +1>(sm, tw, ncols, E);
     } else {
-      plane_rows<E, G::R1, G::R2, -1>(sm, tw, E, ncols);
-      plane_cols<E, G::R1, G::R2, -1>(sm, ncols, tw, E, nrows);
+      plane_rows_padded<E, G::R1, G::R2, -1>(sm, tw, E, ncols);
+      plane_cols_padded<E, G::R1, G::R2, -1>(sm, ncols, tw, E, nrows);
     }
   } else {
     if (dir > 0) {
@@ -695,14 +676,12 @@ __device__ __forceinline__ void plane_fft(float2* sm, int ncols, int nrows, int 
   }
 }
 
-// One plane of one chain after its inverse transforms, in two parts.  plane_update: the kick and the drift, with the
-// state read from srcU / srcQ / srcS (global memory, or shared-memory copies of this plane) and written to Udst / Qc
-// in global memory; the energies' per-thread partials go to pa / pb.  GSRC: srcU / srcQ are in global memory, read with streaming loads (ld.global.cs), as the U and q stores are made; a plane's state is not read
-// again before the next leapfrog step, by which time it has left L2 anyway, and evicting it first keeps T2 and the
-// smaller arrays of the following kernels in L2 (5.97 against 6.04 ms per 64-chain iteration).  The shared-memory
-// copies of the prefetching variant take plain loads: a global-space load of a shared address is an error.
-// plane_finish: the energies' block partials, then the forward transforms and the T2 store.
-template <int E, int NT, bool GSRC>
+// One plane of one chain after its inverse transforms, in two parts.  plane_update: the kick and the drift; the
+// energies' per-thread partials go to pa / pb.  The state is read and written with streaming accesses (ld / st.global.cs):
+// a plane's state is not read again before the next leapfrog step, by which time it has left L2 anyway, and evicting it
+// first keeps T2 and the smaller arrays of the following kernels in L2.  plane_finish: the energies' block partials, then
+// the forward transforms and the T2 store.
+template <int E, int NT>
 __device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, const ChainState& st, int z, bool first, bool last, int flags,
                                              const float2* srcU, const float2* srcQ, const float* srcS,
                                              float2* Udst, float2* Qc, double& pa_out, double& pb_out) {
@@ -732,13 +711,8 @@ __device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, con
     for (int b = 0; b < B; b++) {
       const int e = e0 + b * NT;
       if (e < TOTAL) {
-        if constexpr (GSRC) {
-          u4v[b] = __ldcs(gU + e);
-          q4v[b] = __ldcs(gQ + e);
-        } else {
-          u4v[b] = gU[e];
-          q4v[b] = gQ[e];
-        }
+        u4v[b] = __ldcs(gU + e);
+        q4v[b] = __ldcs(gQ + e);
         s2v[b] = gS[e];
       }
     }
@@ -838,15 +812,14 @@ __device__ __forceinline__ void plane_load_box(float2* sm, const float2* __restr
   }
 }
 
-template <int E, bool PREFETCH>
-__global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETCH>::MINB) k_xyplane(DevVolume v, DevChains ch, int step, int flags,
-                                                                       const float2* __restrict__ tw) {
+template <int E, bool WIDE>
+__global__ void __launch_bounds__(SquareCfg<WIDE>::NT, SquareCfg<WIDE>::MINB) k_plane_square(DevVolume v, DevChains ch, int step, int flags,
+                                                              const float2* __restrict__ tw) {
   grid_dep_wait();
-  constexpr int NT = PlaneCfg<E, PREFETCH>::NT;
-  extern __shared__ __align__(128) unsigned char smraw[];
+  constexpr int NT = SquareCfg<WIDE>::NT;
+  extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double red[NT / 32];
-  const PlaneLayout Ly = plane_layout(E, PlaneGeom<E>::SIZE, PREFETCH);
-  float2* sm = reinterpret_cast<float2*>(smraw + Ly.plane_off);
+  float2* sm = reinterpret_cast<float2*>(smraw);
   const int c = blockIdx.y, z = blockIdx.x;
   const ChainState& st = ch.st[c];
   const int Lc = st.L_cur;
@@ -871,43 +844,188 @@ __global__ void __launch_bounds__(PlaneCfg<E, PREFETCH>::NT, PlaneCfg<E, PREFETC
   // 64^2 planes x 64 chains)
   __shared__ float2 twE[E];
   for (int i = tid; i < E; i += NT) twE[i] = tw[tw_offset(E) + i];
-  const float2* srcU = Usrc;
-  const float2* srcQ = Qc;
-  uint64_t* bar = reinterpret_cast<uint64_t*>(smraw);
-  if (!PREFETCH && (flags & XF_L2_PREFETCH) && tid == 0) {
+  if ((flags & XF_L2_PREFETCH) && tid == 0) {
     bulk_prefetch_l2(Usrc, E * E * 8);
     bulk_prefetch_l2(Qc, E * E * 8);
     bulk_prefetch_l2(Sg, E * E * 4);
   }
-  if constexpr (PREFETCH) {
-    // U and q only: 1/lambda is one array shared by every chain and stays in L2
-    srcU = reinterpret_cast<const float2*>(smraw + Ly.u_off);
-    srcQ = reinterpret_cast<const float2*>(smraw + Ly.q_off);
-    if (tid == 0) {
-      mbar_init(bar, 1);
-      mbar_fence_init();
-      const uint32_t bu = E * E * 8;
-      mbar_arrive_expect_tx(bar, 2 * bu);
-      bulk_g2s(smraw + Ly.u_off, Usrc, bu, bar);
-      bulk_g2s(smraw + Ly.q_off, Qc, bu, bar);
-    }
-  }
   plane_load_box<E, NT>(sm, T, bx, by);
   __syncthreads();
   plane_fft<E>(sm, bx, by, +1, twE);
-  if constexpr (PREFETCH) {
-    const bool ok = mbar_wait_bounded(bar, 0);
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) {
-        atomicExch(ch.err, 1);
-        mbar_wait_bounded(bar, 0, 500000000ull);
-      }
-      return;
-    }
-  }
   double pa, pb;
-  plane_update<E, NT, !PREFETCH>(sm, v, st, z, first, last, flags, srcU, srcQ, Sg, Udst, Qc, pa, pb);
+  plane_update<E, NT>(sm, v, st, z, first, last, flags, Usrc, Qc, Sg, Udst, Qc, pa, pb);
   plane_finish<E, NT>(sm, ch, c, z, first, last, pa, pb, T, bx, by, twE, red);
+}
+
+// ----------------------------------------------------------------- xy-plane kernel
+// The leapfrog update fused with the y and x transforms of one z-plane of one
+// chain (E0, E1 <= 128), one block per (z-plane, chain):
+//   T2[c][z][y < by][x < bx] --inverse y (columns x < bx)--> T[y < E1][x < bx];
+//   per row y: inverse x, kick / drift as in k_xline, forward x --> T[y][x < bx];
+//   --forward y (y < by)--> T2.
+// Only the box's columns of the plane are ever held (E1 x bx); a row's E0 points
+// are in registers between its transforms (row_inverse, row_forward), and a warp
+// takes its rows through all three steps without a block barrier, so that one
+// warp's state is on its way while another transforms (L2 is asked for all of the
+// block's state at entry).  Used for planes with an axis of 128, where a whole plane
+// would leave room for one block on an SM, and for planes that are not square,
+// which otherwise go through separate y passes; the tuner tries it on the others.
+// Measured: 16 chains on 128^3 177 us (whole plane in shared memory, 512
+// threads: 246; x-line kernel with its y passes 190 + 61); 12 chains on 128x64x32 18.7 us
+// (x-line 17.5 + 8.2); 64 chains on 64^3 87 us (k_plane_square 68). It is bound
+// by the L1 pipe (77 %): bank conflicts of the exchanges and the state's runs of
+// 16 LN bytes.  Loading a row's whole state before its inverse transform was slower
+// (128^3: 222 us: it spills at 128 registers).
+// WIDE: 512 threads with all the registers, for chain sets of at most a plane per SM (4 chains on 128x128x64: 21.4 us,
+// 27.9 with the narrow blocks).
+template <int E0, int E1, bool WIDE>
+struct PlaneCfg {
+  static constexpr int NT = WIDE ? 512 : 256;
+  static constexpr int MINB = WIDE ? 1 : ((E0 > 64 || E1 > 64) ? 2 : 3);  // blocks per SM the register budget targets
+  static constexpr int ROW_ELEMS = (NT / 32) * RowPlan<E0>::ROWS * RowPlan<E0>::RP;
+};
+// Shared memory of a block (complex elements): the T array, then the warps' row buffers.
+template <int E0, int E1>
+__host__ __device__ constexpr int plane_box_elems(int bx) { return (E1 * row_pitch<E0>(bx) + 1) / 2 * 2; }
+
+template <int E0, int E1, bool WIDE>
+__global__ void __launch_bounds__(PlaneCfg<E0, E1, WIDE>::NT, PlaneCfg<E0, E1, WIDE>::MINB)
+    k_xyplane(DevVolume v, DevChains ch, int step, int flags, const float2* __restrict__ tw) {
+  grid_dep_wait();
+  using Cfg = PlaneCfg<E0, E1, WIDE>;
+  using PX = RowPlan<E0>;
+  constexpr int NT = Cfg::NT, RP = PX::RP, RA = PX::RA, RB = PX::RB, ROWS = PX::ROWS;
+  constexpr int PAIRS = RA / 2, UB = PAIRS <= 4 || WIDE ? 4 : 2;  // pairs of the state asked for together
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ double red[NT / 32];
+  // the twiddles in shared memory: the stages load a lane's twiddles again for every line, and as global loads (L1
+  // hits) they were most of the kernel's load instructions
+  __shared__ float2 tw0[E0], tw1[E1];
+  const int c = blockIdx.y, z = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const ChainState& st = ch.st[c];
+  const int Lc = st.L_cur;
+  if (step > Lc) return;
+  constexpr int PLANE = E0 * E1;
+  const int bx = v.bx, by = v.by;
+  // the block's plane of the state and of T2 lie in their arrays (checked builds)
+  if (!in_bounds((long long)(z + 1) * PLANE - 1, v.NH, ch.err) || !in_bounds((long long)(z + 1) * by * bx - 1, ch.t2_stride, ch.err))
+    return;
+  const bool first = step == 0, last = step == Lc, fixed = (flags & XF_FIXED_MOMENTUM) != 0;
+  const bool write_q = !last || (flags & XF_WRITE_Q_LAST);
+  const float eps = st.eps_cur, sh = st.sh, keps = ((first || last) ? 0.5f : 1.0f) * eps;
+  const int acc = st.acc;
+  const long long NH = v.NH, at_z = (long long)z * PLANE;
+  const float2* Usrc = ch.U + ((long long)c * 2 + (first ? acc : (acc ^ 1))) * NH + at_z;
+  float2* Udst = ch.U + ((long long)c * 2 + (acc ^ 1)) * NH + at_z;
+  float2* Qc = ch.Q + (long long)c * NH + at_z;
+  const float* Sg = v.sinv + at_z;
+  float2* T = ch.T2 + (long long)c * ch.t2_stride + (long long)z * by * bx;
+  if ((flags & XF_L2_PREFETCH) && tid == 0) {
+    bulk_prefetch_l2(Usrc, PLANE * 8);
+    bulk_prefetch_l2(Qc, PLANE * 8);
+    bulk_prefetch_l2(Sg, PLANE * 4);
+  }
+  for (int i = tid; i < E0; i += NT) tw0[i] = tw[tw_offset(E0) + i];
+  for (int i = tid; i < E1; i += NT) tw1[i] = tw[tw_offset(E1) + i];
+  const int pitch = row_pitch<E0>(bx);
+  float2* box = reinterpret_cast<float2*>(smraw);
+  // the box in pairs of x-adjacent points (bx is even); the last read of this T2 plane before the next inverse z pass
+  const int hx = bx / 2;
+  const uint32_t mb = box_div_magic(hx);
+  for (int e = tid; e < by * hx; e += NT) {
+    const int y = hx == 1 ? e : (int)__umulhi((uint32_t)e, mb), x = 2 * (e - y * hx);
+    const float4 t = __ldcs(reinterpret_cast<const float4*>(T) + e);
+    float2* d = box + y * pitch + x;
+    d[0] = make_float2(t.x, t.y);
+    d[1] = make_float2(t.z, t.w);
+  }
+  __syncthreads();
+  plane_cols<E1, +1>(box, pitch, bx, tw1, by, E1);
+  __syncthreads();
+
+  const int r = lane / PX::LN, b = lane % PX::LN;
+  float2* row = box + plane_box_elems<E0, E1>(bx) + (warp * ROWS + r) * RP;
+  double pa = 0.0, pb = 0.0;
+#pragma unroll 1
+  for (int y0 = warp * ROWS; y0 < E1; y0 += (NT / 32) * ROWS) {  // E1 is a multiple of ROWS
+    const int y = y0 + r;
+    // the lane's pairs of points, UB at a time: pair i = (mm, k) is points p(2 mm) + RA k and the next
+    auto pair_at = [&](int i) { return (y * E0 + PX::butterfly(b, 2 * (i / RB)) + RA * (i % RB)) / 2; };
+    float4 u4v[UB], q4v[UB];
+    float2 s2v[UB];
+    float2 e[PX::NBF][RB];
+    row_inverse<E0>(box + y * pitch, bx, row, b, tw0, e);
+#pragma unroll
+    for (int i0 = 0; i0 < PAIRS; i0 += UB) {
+#pragma unroll
+      for (int i = 0; i < UB; i++) {
+        const int at = pair_at(i0 + i);
+        u4v[i] = __ldcs(reinterpret_cast<const float4*>(Usrc) + at);
+        q4v[i] = __ldcs(reinterpret_cast<const float4*>(Qc) + at);
+        s2v[i] = __ldg(reinterpret_cast<const float2*>(Sg) + at);
+      }
+#pragma unroll
+      for (int i = 0; i < UB; i++) {
+        const int at = pair_at(i0 + i), mm = (i0 + i) / RB, k = (i0 + i) % RB;
+        float2 uo[2], qo[2];
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+          const float2 u = m == 0 ? make_float2(u4v[i].x, u4v[i].y) : make_float2(u4v[i].z, u4v[i].w);
+          const float s = m == 0 ? s2v[i].x : s2v[i].y;
+          const bool live = s > 0.0f;
+          const float lm = s + sh;  // lambda_m = 1/lambda + sigma_h^-2 (MultiResParameters.h:735-738)
+          float2 q = m == 0 ? make_float2(q4v[i].x, q4v[i].y) : make_float2(q4v[i].z, q4v[i].w);
+          if (first && live) {  // the kinetic energy of a drawn momentum is k_momentum's sum |w|^2
+            if (fixed) pa += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+            pb += (double)(u.x * u.x + u.y * u.y) * (double)s;
+          }
+          const float2 g = e[2 * mm + m][k];
+          float2 gt = g;
+          if (live) {
+            gt.x = fmaf(-u.x, s, g.x);
+            gt.y = fmaf(-u.y, s, g.y);
+          }
+          q.x = fmaf(keps, gt.x, q.x);
+          q.y = fmaf(keps, gt.y, q.y);
+          float2 un = u;
+          if (last) {
+            if (live && !first) {  // first and last: an evaluation step, energies at mu only
+              pa += (double)(u.x * u.x + u.y * u.y) * (double)s;
+              pb += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+            }
+          } else if (live) {
+            const float f = eps / lm;
+            un.x = fmaf(f, q.x, u.x);
+            un.y = fmaf(f, q.y, u.y);
+          }
+          uo[m] = un;
+          qo[m] = q;
+          e[2 * mm + m][k] = un;
+        }
+        // streaming loads and stores of the state: it is not read again before the next leapfrog step, by which time
+        // it has left L2 on large chain sets; evicting it first keeps T2 and the following kernels' arrays there
+        if (write_q) __stcs(reinterpret_cast<float4*>(Qc) + at, make_float4(qo[0].x, qo[0].y, qo[1].x, qo[1].y));
+        if (!last) __stcs(reinterpret_cast<float4*>(Udst) + at, make_float4(uo[0].x, uo[0].y, uo[1].x, uo[1].y));
+      }
+    }
+    if (!last) row_forward<E0>(e, row, b, tw0, box + y * pitch, bx);
+  }
+  if (first || last) {
+    const double wt = plane_weight(z, v.E2);
+    const double ta = block_sum(wt * pa, red);
+    if (tid == 0) ch.part[((long long)c * NSLOT + (first ? SL_E0 : SL_LPL)) * ch.maxblk + z] = ta;
+    const double tb = block_sum(wt * pb, red);
+    if (tid == 0) ch.part[((long long)c * NSLOT + (first ? SL_LP0 : SL_KL)) * ch.maxblk + z] = tb;
+  }
+  if (last) return;
+  __syncthreads();
+  plane_cols<E1, -1>(box, pitch, bx, tw1, E1, by);
+  __syncthreads();
+  for (int e = tid; e < by * hx; e += NT) {
+    const int y = hx == 1 ? e : (int)__umulhi((uint32_t)e, mb), x = 2 * (e - y * hx);
+    const float2* d = box + y * pitch + x;
+    reinterpret_cast<float4*>(T)[e] = make_float4(d[0].x, d[0].y, d[1].x, d[1].y);
+  }
 }
 
 // ----------------------------------------------------------------- per-iteration scalars
