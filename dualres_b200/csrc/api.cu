@@ -517,7 +517,7 @@ static void kriging_solve_device(HostVolume& hv, int device, cudaStream_t st) {
   auto upload = [&](void* dst, const void* src, size_t bytes) {
     if (bytes) CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
   };
-  fill_vector<double> w(P.col.size());  // every entry comes back from the device (zeroed there)
+  fill_vector<float> w(P.col.size());  // every entry comes back from the device (zeroed there)
   std::vector<char> keep(nrows, 1);
   std::vector<int> status(nrows, KR_OK);
   std::vector<int> dup_of(nrows, -1);
@@ -608,8 +608,9 @@ static void kriging_solve_device(HostVolume& hv, int device, cudaStream_t st) {
       upload(d_tt, task_route.data(), sizeof(int) * ntasks);
       int* d_cnt = (int*)dalloc(sizeof(int));
       CK(cudaMemsetAsync(d_cnt, 0, sizeof(int), st));
-      double* d_w = (double*)dalloc(sizeof(double) * w.size());
-      CK(cudaMemsetAsync(d_w, 0, sizeof(double) * w.size(), st));
+      double* d_x = (double*)dalloc(sizeof(double) * w.size());
+      float* d_w = (float*)dalloc(sizeof(float) * w.size());
+      CK(cudaMemsetAsync(d_w, 0, sizeof(float) * w.size(), st));
       int* d_status = (int*)dalloc(sizeof(int) * nrows);
       CK(cudaMemsetAsync(d_status, 0, sizeof(int) * nrows, st));
       double* d_scr = (double*)dalloc(sizeof(double) * slot * grid);
@@ -620,6 +621,7 @@ static void kriging_solve_device(HostVolume& hv, int device, cudaStream_t st) {
       a.task_route = d_tt;
       a.ntasks = ntasks;
       a.counter = d_cnt;
+      a.x = d_x;
       a.w = d_w;
       a.status = d_status;
       a.scratch = d_scr;
@@ -629,9 +631,9 @@ static void kriging_solve_device(HostVolume& hv, int device, cudaStream_t st) {
         CK(cudaStreamSynchronize(st));
         tr_rows.next("kriging: row-solve kernel + download");
       }
-      k_kriging_rows<<<grid, KR_NT, sizeof(KrigSmem), st>>>(a);
+      k_kriging_rows<<<grid, KR_RT, sizeof(KrigSmem), st>>>(a);
       CK_LAUNCH();
-      CK(cudaMemcpyAsync(w.data(), d_w, sizeof(double) * w.size(), cudaMemcpyDeviceToHost, st));
+      CK(cudaMemcpyAsync(w.data(), d_w, sizeof(float) * w.size(), cudaMemcpyDeviceToHost, st));
       CK(cudaMemcpyAsync(status.data(), d_status, sizeof(int) * nrows, cudaMemcpyDeviceToHost, st));
       CK(cudaStreamSynchronize(st));
     }
@@ -663,7 +665,8 @@ static void kriging_solve_device(HostVolume& hv, int device, cudaStream_t st) {
   for (int i = 0; i < (int)redo.size(); i++) {
     std::vector<double> x;
     const int ri = redo[i];
-    if (kriging_solve_row_host(P, ri, &x)) std::copy(x.begin(), x.end(), w.begin() + P.row_start[ri]);
+    if (kriging_solve_row_host(P, ri, &x))
+      std::transform(x.begin(), x.end(), w.begin() + P.row_start[ri], [](double v) { return (float)v; });
     else keep[ri] = 0;
   }
   for (int ri = 0; ri < nrows; ri++) {
@@ -1145,9 +1148,9 @@ static void init_chain_states(Chainset* S) {
 }
 
 // ---------------------------------------------------------------- autotuning
-// Candidate update paths for an embedding: the fused plane kernel (square x/y
-// planes whose padded layout fits shared memory), the same with bulk prefetch
-// of the state planes, and the x-line kernel with separate y passes (always).
+// Candidate update paths for an embedding: the fused plane kernels (square
+// x/y planes up to 64 whole in shared memory; planes with sides 16 to 128 with
+// their rows in registers) and the x-line kernel with separate y passes (always).
 // ---------------------------------------------------------------- tensor-core kriging products
 static void tc_upload(Volume* V, const TcPlanHost& P, const float* val, int nnz, int n_rows, int n_cols,
                       DevTcMatrix* M) {

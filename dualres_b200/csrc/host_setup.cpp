@@ -487,7 +487,8 @@ void kriging_solve_host(const KrigingPlan& plan, std::vector<int>* rowptr, fill_
   kriging_assemble(plan, flat.data(), keep, rowptr, col, val);
 }
 
-void kriging_assemble(const KrigingPlan& plan, const double* w, const std::vector<char>& keep,
+template <class T>
+void kriging_assemble(const KrigingPlan& plan, const T* w, const std::vector<char>& keep,
                       std::vector<int>* rowptr, fill_vector<int>* col, fill_vector<float>* val) {
   rowptr->assign(plan.nrows + 1, 0);
   for (int ri = 0; ri < plan.nrows; ri++) {
@@ -506,6 +507,10 @@ void kriging_assemble(const KrigingPlan& plan, const double* w, const std::vecto
     }
   }
 }
+template void kriging_assemble(const KrigingPlan&, const double*, const std::vector<char>&, std::vector<int>*,
+                               fill_vector<int>*, fill_vector<float>*);
+template void kriging_assemble(const KrigingPlan&, const float*, const std::vector<char>&, std::vector<int>*,
+                               fill_vector<int>*, fill_vector<float>*);
 
 int kriging_build(const float* hr, int nx, int ny, int nz, const float* Qhr, const float* sr, int sx, int sy, int sz,
                   const float* Qsr, const float* theta, float radius, std::vector<int>* rowptr, std::vector<int>* col,

@@ -96,7 +96,8 @@ void kriging_solve_host(const KrigingPlan& plan, std::vector<int>* rowptr, fill_
 // false when its weight sum is NaN.
 bool kriging_solve_row_host(const KrigingPlan& plan, int ri, std::vector<double>* x);
 // CSR from per-candidate weights; rows with keep = 0 are emptied (NaN weight sums).
-void kriging_assemble(const KrigingPlan& plan, const double* w, const std::vector<char>& keep,
+template <class T>
+void kriging_assemble(const KrigingPlan& plan, const T* w, const std::vector<char>& keep,
                       std::vector<int>* rowptr, fill_vector<int>* col, fill_vector<float>* val);
 
 // Kriging CSR of kriging_matrix.h:148-343 (exposed for tests through the volume).
