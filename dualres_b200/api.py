@@ -378,6 +378,8 @@ class MultiResParameters:
         a = np.ascontiguousarray(x, dtype=np.complex64).reshape(self.data.shape)
         return a
 
+    # "plane+prefetch": the plane kernel with its rows in registers on a shape where "plane" keeps the whole plane in
+    # shared memory (the name is the one callers know)
     PATHS = ("plane", "plane+prefetch", "lines")
 
     def config(self):
@@ -496,9 +498,10 @@ def debug_dual_averaging(burnin, nsave, thin, L, starting_eps, mhtarget, rates, 
     return e, s
 
 
-KERNEL_NAMES = ["state update (k_xyplane when E0 == E1 <= 128, else k_xline)", "forward y pass (k_pass)", "forward z pass + gather (k_pass)",
-                "W product (k_tc_product + k_tc_finish from 16 chains, else k_spmv_w)",
-                "W^T product (k_tc_product + k_tc_finish from 16 chains, else k_spmv_wt)", "inverse z pass (k_pass)",
+KERNEL_NAMES = ["state update (k_plane_square / k_xyplane where a plane kernel fits, else k_xline)", "forward y pass (k_pass)",
+                "forward z pass + gather (k_zfwd)",
+                "W product (k_tc_product + k_tc_finish from 16 chains, else k_row_product)",
+                "W^T product (k_tc_product + k_tc_finish from 16 chains, else k_row_product)", "inverse z pass (k_zinv)",
                 "inverse y pass (k_pass)"]
 
 

@@ -145,8 +145,11 @@ struct DeviceTables {
 static std::mutex g_dev_mtx;
 static DeviceTables g_dev[64];
 
+// Raises a kernel's limit of dynamic shared memory.  Up to 32 KB the default of 48 KB suffices (static memory included),
+// and asking would load the kernel: loading only what a process launches makes its first call 10 ms shorter.
 template <class K>
 static void set_smem(K* kernel, int bytes) {
+  if (bytes <= (32 << 10)) return;
   CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
 }
 

@@ -1,9 +1,8 @@
 // Bulk asynchronous copies (1D TMA, cp.async.bulk) and mbarriers for sm_100a.
 //
-// Global -> shared copies complete on an mbarrier (transaction bytes);
-// shared -> global copies are tracked with bulk groups.  Sources,
-// destinations and sizes must be multiples of 16 bytes.  These are plain
-// CTA-local copies: no cluster multicast is used anywhere.
+// Global -> shared copies complete on an mbarrier (transaction bytes).
+// Sources, destinations and sizes must be multiples of 16 bytes.  These are
+// plain CTA-local copies: no cluster multicast is used anywhere.
 #pragma once
 
 #include <stdint.h>
@@ -76,23 +75,12 @@ __device__ __forceinline__ void tma_gather4(void* dst, const void* tmap, int x, 
       : "memory");
 }
 
-__device__ __forceinline__ void bulk_s2g(void* dst, const void* src, uint32_t bytes) {
-  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_addr(src)),
-               "r"(bytes)
-               : "memory");
-}
-
 // Asks L2 to fetch [src, src + bytes) from global memory ahead of its use; nothing to wait for (16-byte aligned
 // address, size a multiple of 16).
 __device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-// Shared memory of every committed store may be reused.
-__device__ __forceinline__ void bulk_wait_read_all() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// Every committed store has completed.
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Orders this thread's generic-proxy shared-memory writes before later async-proxy reads.
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 

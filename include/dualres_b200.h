@@ -161,12 +161,14 @@ int dr_samples_get(dr_chainset* cs, int chain, float* samples, int max_saved, in
 int dr_sample_records_get(dr_chainset* cs, int chain, double* rec, int max_saved, int* n_saved);
 void dr_chainset_destroy(dr_chainset* cs);
 /* The configuration the chain set runs (no reference counterpart): update path
- * (0 fused x/y plane kernel, 1 the same with bulk prefetch of the state planes,
- * 2 x-line kernel with separate y passes), kriging-product blocks per SM, the
+ * (0 fused x/y plane kernel, 1 its variant with the rows in registers on a shape
+ * where 0 keeps the whole plane in shared memory, 2 x-line kernel with separate y
+ * passes), kriging-product blocks per SM, the
  * iteration time measured when the shape was tuned (0 when it was not), and
  * whether the kriging products run on the tensor cores (1; 2 when W^T's chain
- * vectors arrive by TMA row gathers) or as CSR products (0).  At creation the update paths are timed on a scratch chain set of the
- * same shape (with the tensor-core products where available), then the other
+ * vectors arrive by TMA row gathers) or over groups of rows (0).  At creation the
+ * update paths are timed on a scratch chain set of the same shape (with the
+ * tensor-core products where available), then the other
  * product choices on the fastest path, and the fastest is kept for the process;
  * DRB_AUTOTUNE=0 turns this off, DRB_NO_PLANE / DRB_PLANE_PREFETCH force a
  * path, DRB_TC_PRODUCTS=0 / 1 the products.  Any output may be NULL. */
