@@ -3113,18 +3113,23 @@ int dr_mce_summary(const float* img, int nx, int ny, int nz, const float* qform,
     float* d_rows = (float*)dalloc(sizeof(float) * (size_t)(rows + 1) * g.pitch);
     uint32_t* d_bits = (uint32_t*)dalloc(sizeof(uint32_t) * (size_t)(rows + 1) * g.bw);
     int* d_any = (int*)dalloc(sizeof(int) * (rows + 1));
+    int* d_inf = (int*)dalloc(sizeof(int));
     MceTask* d_tasks = (MceTask*)dalloc(sizeof(MceTask) * n_tasks);
-    MceSums* d_part = (MceSums*)dalloc(sizeof(MceSums) * (size_t)n_slabs * n_off);
+    MceSums* d_part = (MceSums*)dalloc(sizeof(MceSums) * (size_t)(n_slabs + 1) * n_off);
     float* d_cov = (float*)dalloc(sizeof(float) * n_off);
     int* d_np = (int*)dalloc(sizeof(int) * n_off);
     double* d_sums = sums ? (double*)dalloc(sizeof(double) * 3 * n_off) : nullptr;
     CK(cudaMemcpyAsync(d_img, img, sizeof(float) * nvox, cudaMemcpyHostToDevice, st));
     CK(cudaMemcpyAsync(d_tasks, tasks.data(), sizeof(MceTask) * n_tasks, cudaMemcpyHostToDevice, st));
-    k_mce_rows<<<rows + 1, 32, 0, st>>>(d_img, g, d_rows, d_bits, d_any);
+    CK(cudaMemsetAsync(d_inf, 0, sizeof(int), st));
+    k_mce_rows<<<rows + 1, 32, 0, st>>>(d_img, g, d_rows, d_bits, d_any, d_inf);
     CK_LAUNCH();
     k_mce_pairs<<<dim3(n_slabs, tb), MCE_THREADS, 0, st>>>(d_rows, d_bits, d_any, g, d_tasks, n_tasks, n_off, d_part);
     CK_LAUNCH();
-    k_mce_finish<<<cdiv_i(n_off, 256), 256, 0, st>>>(d_part, n_slabs, n_off, d_cov, d_np, d_sums);
+    k_mce_infinite<<<cdiv_i(n_tasks * MCE_LAGS, 256), 256, 0, st>>>(d_img, d_any, d_inf, g, d_tasks, n_tasks,
+                                                                    d_part + (size_t)n_slabs * n_off);
+    CK_LAUNCH();
+    k_mce_finish<<<cdiv_i(n_off, 256), 256, 0, st>>>(d_part, n_slabs + 1, n_off, d_cov, d_np, d_sums);
     CK_LAUNCH();
     CK(cudaMemcpyAsync(covariance, d_cov, sizeof(float) * n_off, cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(npairs, d_np, sizeof(int) * n_off, cudaMemcpyDeviceToHost, st));

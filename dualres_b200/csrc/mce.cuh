@@ -12,7 +12,9 @@
 // values that slides along the row in registers, so 96 FMAs take one 16-byte
 // load of each row and eight conversions.  Masked values are zero and masks
 // are factors 0 or 1, so that nothing branches; the counts come from bit rows by
-// popcount.  Rows are padded with zeros (dx0 is a multiple of 4: every load is
+// popcount.  Infinite voxels would meet those zeros (0 * inf is NaN), so the rows
+// hold 0 in their place and k_mce_infinite adds their pairs; without any it only
+// writes its zeros (2 us).  Rows are padded with zeros (dx0 is a multiple of 4: every load is
 // aligned and none is tested), rows outside the grid are a row of zeros, and x
 // rows without data are skipped.  Slabs interleave the rows, which balances
 // them; a second kernel adds the slabs in order, so results do not depend on
@@ -42,26 +44,31 @@ struct MceRows {
   int nx, ny, nz, pitch, bw;
 };
 
+// any[r]: 0 without data, 2 with an infinite voxel (which also sets *infinite), else 1.
 __global__ void k_mce_rows(const float* __restrict__ img, MceRows g, float* __restrict__ rows, uint32_t* __restrict__ bits,
-                           int* __restrict__ any) {
+                           int* __restrict__ any, int* __restrict__ infinite) {
   const int r = blockIdx.x, lane = threadIdx.x;  // one warp per row
   const bool real = r < g.ny * g.nz;
   float* row = rows + (long long)r * g.pitch;
   for (int i = lane; i < g.pitch; i += 32) {
     const int x = i - MCE_FRONT;
     float v = real && x >= 0 && x < g.nx ? img[(long long)r * g.nx + x] : 0.f;
-    if (isnan(v)) v = 0.f;
+    if (!isfinite(v)) v = 0.f;
     row[i] = v;
   }
-  uint32_t some = 0;
+  uint32_t some = 0, inf = 0;
   for (int q = 0; q < g.bw; q++) {
     const int x = 32 * (q - 1) + lane;
     const float v = real && x >= 0 && x < g.nx ? img[(long long)r * g.nx + x] : 0.f;
     const uint32_t b = __ballot_sync(0xffffffffu, !isnan(v) && v != 0.f);
     if (lane == 0) bits[(long long)r * g.bw + q] = b;
     some |= b;
+    inf |= __ballot_sync(0xffffffffu, isinf(v));
   }
-  if (lane == 0) any[r] = some != 0;
+  if (lane == 0) {
+    any[r] = inf != 0 ? 2 : some != 0;
+    if (inf != 0) *infinite = 1;
+  }
 }
 
 __global__ void __launch_bounds__(MCE_THREADS) k_mce_pairs(const float* __restrict__ rows, const uint32_t* __restrict__ bits,
@@ -133,6 +140,41 @@ __global__ void __launch_bounds__(MCE_THREADS) k_mce_pairs(const float* __restri
     const int o = T->out[l];
     if (o >= 0) part[(long long)blockIdx.x * n_off + o] = MceSums{sxy[l], sx[l], sy[l], n[l]};
   }
+}
+
+// The pairs of infinite voxels, as one more slab: a thread takes one offset p and, for each infinite voxel v in the image's order,
+// the pairs (v, v + p) and, unless its other voxel is infinite too (and counts it), (v - p, v).  The counts are k_mce_pairs'.
+__global__ void k_mce_infinite(const float* __restrict__ img, const int* __restrict__ any, const int* __restrict__ infinite,
+                               MceRows g, const MceTask* __restrict__ tasks, int n_tasks, MceSums* __restrict__ part) {
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) / MCE_LAGS, l = threadIdx.x % MCE_LAGS;
+  if (t >= n_tasks || tasks[t].out[l] < 0) return;
+  MceSums s{0.0, 0.0, 0.0, 0};
+  if (*infinite) {
+    const int p[3] = {tasks[t].dx0 + l, tasks[t].dy, tasks[t].dz};
+    // the value at (x, y, z), 0 where it is masked or outside the grid
+    auto value = [&](int x, int y, int z) {
+      if (x < 0 || x >= g.nx || y < 0 || y >= g.ny || z < 0 || z >= g.nz) return 0.f;
+      const float v = img[((long long)z * g.ny + y) * g.nx + x];
+      return isnan(v) ? 0.f : v;
+    };
+    auto add = [&](float x, float y) {
+      s.sxy += (double)x * (double)y;
+      s.sx += (double)x;
+      s.sy += (double)y;
+    };
+    for (int r = 0; r < g.ny * g.nz; r++) {
+      if (any[r] != 2) continue;
+      const int y = r % g.ny, z = r / g.ny;
+      for (int x = 0; x < g.nx; x++) {
+        const float v = img[(long long)r * g.nx + x];
+        if (!isinf(v)) continue;
+        const float b = value(x + p[0], y + p[1], z + p[2]), a = value(x - p[0], y - p[1], z - p[2]);
+        if (b != 0.f) add(v, b);
+        if (a != 0.f && !isinf(a)) add(a, v);
+      }
+    }
+  }
+  part[tasks[t].out[l]] = s;
 }
 
 // Slab sums in order; covariance (sum_xy - sum_x sum_y / n) / (n - 1) for n > 1, else 0.
