@@ -28,6 +28,7 @@ namespace drb {
 
 constexpr int MCE_THREADS = 128;
 constexpr int MCE_LAGS = 8;
+constexpr int MCE_REACH = 25;  // largest |component| of an offset (perturbation_matrix.h:19-109)
 constexpr int MCE_FRONT = 32, MCE_BACK = 40;  // zeros before and after a row: dx0 >= -20, dx0 + 7 <= 27
 
 struct MceSums {
