@@ -1244,9 +1244,9 @@ __global__ void k_base(double2* base, int E0, int E1, int E2, float q00, float q
 }
 
 // S = {Re lambda <= 0} (MultiResParameters.h:258-262); sinv = 1/Re lambda on live modes.  The base is even in every
-// axis, so lambda(k) and lambda(-k) are the same number; the transform leaves them a rounding apart.  sinv is formed
-// from their mean, which both get bit for bit: a Hermitian field stays Hermitian under the sampler's element-wise
-// steps.  (lam_re and n_S report the transform's own values.)
+// axis, so lambda(k) and lambda(-k) are the same number; the transform leaves them a rounding apart.  S and sinv are
+// formed from their mean, which both get bit for bit: a Hermitian field stays Hermitian under the sampler's element-wise
+// steps, and n_S counts the modes that are masked.  (lam_re reports the transform's own values.)
 __global__ void k_spectrum(const double2* lam, float* sinv, double* lam_re, int E0, int E1, int E2, int* n_S) {
   const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (long long)E0 * E1 * E2) return;
@@ -1254,7 +1254,7 @@ __global__ void k_spectrum(const double2* lam, float* sinv, double* lam_re, int 
   const long long j = ((long long)(z == 0 ? 0 : E2 - z) * E1 + (y == 0 ? 0 : E1 - y)) * E0 + (x == 0 ? 0 : E0 - x);
   const double re = lam[i].x, sym = 0.5 * (re + lam[j].x);
   lam_re[i] = re;
-  if (re <= 0.0) atomicAdd(n_S, 1);
+  if (sym <= 0.0) atomicAdd(n_S, 1);
   sinv[i] = sym > 0.0 ? (float)(1.0 / sym) : -1.0f;
 }
 
