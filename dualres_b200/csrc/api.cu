@@ -701,9 +701,9 @@ static void volume_rows(Volume* V, const std::vector<int>& rowptr, const int* co
   d.groups = h.groups();
   d.entries = (long long)h.off.size();
   d.ptr = V->upload(h.ptr);
-  d.base = V->upload(h.base);
-  d.off = V->upload(h.off);
-  d.val = V->upload(h.val);
+  d.base = V->upload(h.base) + h.origin / 32;
+  d.off = V->upload(h.off) + h.origin;
+  d.val = V->upload(h.val) + h.origin * ROWP_R;
   CK(cudaStreamSynchronize(V->stream));  // the host arrays are released on return
 }
 

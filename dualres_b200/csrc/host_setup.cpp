@@ -601,9 +601,10 @@ bool row_groups(const std::vector<int>& rowptr, const int* col, const float* val
     first[u + 1] = n;
   }
   for (int u = 0; u < units; u++) first[u + 1] += first[u];
-  if (first[units] > INT_MAX - 4096) return false;
+  if (first[units] > ROWP_MAX_ENTRIES) return false;
+  out->origin = first[units] > INT_MAX - 4096 ? ROWP_ORIGIN : 0;
   const size_t n = (size_t)(first[units] + ROWP_PAD - 1) / ROWP_PAD * ROWP_PAD;
-  out->ptr.assign(G + 1, (int)first[units]);
+  out->ptr.assign(G + 1, (int)(first[units] - out->origin));
   out->base.resize(n / 32);
   out->off.resize(n);
   out->val.resize(n * R);
@@ -621,7 +622,7 @@ bool row_groups(const std::vector<int>& rowptr, const int* col, const float* val
       out->base[k / 32 - 1] = base;
       for (int b = 0; b < 32; b++) out->off[k - 32 + b] = (uint16_t)(cols[b] >= 0 ? cols[b] - base : 0);
     };
-    merge_groups(rowptr, col, val, u * UNIT, std::min(G, (u + 1) * UNIT), put, [&](int g) { out->ptr[g] = (int)k; });
+    merge_groups(rowptr, col, val, u * UNIT, std::min(G, (u + 1) * UNIT), put, [&](int g) { out->ptr[g] = (int)((long long)k - out->origin); });
   }
   const size_t end = (size_t)first[units];  // the padding is brought to L2 with the last entries and never used
   std::fill(out->base.begin() + end / 32, out->base.end(), 0);

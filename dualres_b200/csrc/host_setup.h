@@ -107,13 +107,14 @@ int kriging_build(const float* hr, int nx, int ny, int nz, const float* Qhr, con
 
 // A CSR matrix in groups of ROWP_R consecutive rows over the union of their columns, as DevRowGroups describes it.
 struct RowGroupsHost {
-  std::vector<int> ptr;  // groups + 1
+  std::vector<int> ptr;  // groups + 1, from origin
+  long long origin = 0;  // 0 or ROWP_ORIGIN
   fill_vector<int> base;
   fill_vector<uint16_t> off;
   fill_vector<float> val;
   int groups() const { return (int)ptr.size() - 1; }
 };
-// false when the entries would not be addressable with 32-bit positions.
+// false above ROWP_MAX_ENTRIES entries.
 bool row_groups(const std::vector<int>& rowptr, const int* col, const float* val, RowGroupsHost* out);
 
 // Host part of a dense-tile plan for the tensor-core kriging products: rows
