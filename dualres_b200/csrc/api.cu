@@ -1322,9 +1322,11 @@ static bool autotune_enabled() {
 
 struct TuneKey {
   int dev, E0, E1, E2, bx, by, bz, C, n_h, n_s, L;  // n_h, n_s as tune_bucket()s
+  int row;  // octave of the mean row length of W: the products' cost grows with the kriging radius at equal counts
+  bool tc;  // the tensor-core products were admitted as candidates
   bool operator<(const TuneKey& o) const {
-    return std::tie(dev, E0, E1, E2, bx, by, bz, C, n_h, n_s, L) <
-           std::tie(o.dev, o.E0, o.E1, o.E2, o.bx, o.by, o.bz, o.C, o.n_h, o.n_s, o.L);
+    return std::tie(dev, E0, E1, E2, bx, by, bz, C, n_h, n_s, L, row, tc) <
+           std::tie(o.dev, o.E0, o.E1, o.E2, o.bx, o.by, o.bz, o.C, o.n_h, o.n_s, o.L, o.row, o.tc);
   }
 };
 static std::mutex g_tune_mtx;
@@ -1352,7 +1354,8 @@ static TuneChoice autotune(Volume* V, int C, const dr_hmc_opts* o) {
   const NvtxRange range("chain set: tuning");
   const DevVolume& v = V->dv;
   const TuneKey key{V->device, v.E0, v.E1, v.E2, v.bx, v.by, v.bz, C, tune_bucket(v.n_h), tune_bucket(v.n_s),
-                    o->leapfrog};
+                    o->leapfrog, v.n_s > 0 ? (int)std::lround(std::log2(1.0 + (double)V->hv.w_col.size() / v.n_s)) : -1,
+                    !tc_env_off()};
   {
     std::lock_guard<std::mutex> lk(g_tune_mtx);
     auto it = g_tune.find(key);
