@@ -896,34 +896,35 @@ static void launch_rowp_t(const RowpLaunch& a) {
   else if (a.warps == 8) launch_rowp_k<V, CL, NR, 8, false>(a);
   else launch_rowp_k<V, CL, NR, 4, false>(a);
 }
-// CL lanes of V chains (the largest vector that divides C; up to 4 chains: a lane per entry with all of them, 3 chains in
-// 4 lanes) and NR rounds cover the chains.
+// CL lanes of V chains (the largest vector that divides C) and NR rounds cover the chains: from 5 chains every lane has 4 of them,
+// in rounds of its vector, so that a warp takes as many entries at a time with any count of chains.  (Odd counts with a lane
+// per chain took, W / W^T: 9 chains, 43x23x17 23.3 / 17.7 us, now 9.1 / 9.4; 5 chains, 64x64x48 51.7 / 38.1, now 26.6 / 23.5;
+// 17 chains, 12x10x8 13.3 / 8.5, now 5.5 / 5.4.)
 template <int V>
 static void launch_rowp_v(const RowpLaunch& a) {
   const int lanes = a.ch.C / V;
+  constexpr int NR = 4 / V;
   if (lanes <= 1) return launch_rowp_t<V, 1, 1>(a);
-  if constexpr (V == 4)
-    if (lanes <= 2) return launch_rowp_t<V, 2, 1>(a);
-  if (lanes <= 4) return launch_rowp_t<V, 4, 1>(a);
-  if (lanes <= 8) return launch_rowp_t<V, 8, 1>(a);
-  if (lanes <= 16) return launch_rowp_t<V, 16, 1>(a);
-  if (lanes <= 32) return launch_rowp_t<V, 32, 1>(a);
-  if (lanes <= 64) return launch_rowp_t<V, 32, 2>(a);
-  if constexpr (V <= 2)
-    if (lanes <= 128) return launch_rowp_t<V, 32, 4>(a);
-  if constexpr (V == 1) return launch_rowp_t<V, 32, 8>(a);
+  if constexpr (V == 1)
+    if (lanes <= 3) return launch_rowp_t<1, 4, 1>(a);
+  if (lanes <= 2 * NR) return launch_rowp_t<V, 2, NR>(a);
+  if (lanes <= 4 * NR) return launch_rowp_t<V, 4, NR>(a);
+  if (lanes <= 8 * NR) return launch_rowp_t<V, 8, NR>(a);
+  if (lanes <= 16 * NR) return launch_rowp_t<V, 16, NR>(a);
+  if (lanes <= 32 * NR) return launch_rowp_t<V, 32, NR>(a);
+  return launch_rowp_t<V, 32, 2 * NR>(a);  // up to 256 chains
 }
 static void launch_rowp(const RowpLaunch& a) {
   if (a.ch.C % 4 == 0) launch_rowp_v<4>(a);
   else if (a.ch.C % 2 == 0) launch_rowp_v<2>(a);
   else launch_rowp_v<1>(a);
 }
-// Warps that share a group: one for W^T; for W 8 with up to 2 chains per lane or when the groups are fewer than 8 per SM,
+// Warps that share a group: one for W^T; for W 8 with less than 4 chains per lane or when the groups are fewer than 8 per SM,
 // else 4 (2 chains, 80x80x64: 60 us with 8, 81 with 4; 12 chains, 281 groups: 9.7 and 13.9; 16 chains, 3294 groups: 36.4
-// and 30.7).
+// and 30.7; 5 chains, 64x64x48 at 3.6 mm: 15.7 and 10.3).
 static int rowp_warps(const DevRowGroups& M, const DevChains& ch, bool w, int sms) {
   if (!w) return 1;
-  return (ch.C % 4 != 0 || M.groups < 8 * sms) ? 8 : 4;
+  return (ch.C < 4 || M.groups < 8 * sms) ? 8 : 4;
 }
 // Blocks of a product: at most blocks_per_sm, and no more than are resident together, on every SM.
 static int rowp_blocks(const DevRowGroups& M, const DevVolume& v, const DevChains& ch, bool w, int sms, int blocks_per_sm) {

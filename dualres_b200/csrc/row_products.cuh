@@ -11,8 +11,8 @@
 // rows lie two voxels apart, 1.7 (7.8 bytes); a third and two fifths of the gathers.
 //
 // A warp takes S = 32 / CL entries at a time: CL lanes share an entry, each with
-// V adjacent chains (one vector load) in NR rounds; with 1, 2 or 4 chains every
-// lane has its own entry.  U steps' loads are issued before any is used, and L2
+// V adjacent chains (one vector load) in NR rounds, 4 chains per lane from 5 chains;
+// with 1, 2 or 4 chains every lane has its own entry.  U steps' loads are issued before any is used, and L2
 // is asked for the next group's entries meanwhile.  SW warps share a group of
 // W, whose groups are few and long; a group of W^T has a warp of its own.  The
 // sums are reduced over the lanes by halving exchanges (the rows are divided
