@@ -55,6 +55,8 @@ __device__ __forceinline__ int hmc_steps(const ChainState& h) {  // :172-179
 __device__ __forceinline__ int hmc_save_iteration(const ChainState& h) {  // :158-161
   return (h.iteration > h.burnin) && ((h.iteration - h.burnin) % h.thin == 0);
 }
+// During the burn-in the step size follows the rate min(1, R): where log R lies a few units below zero, its rounding (1e-4 to
+// 1e-3) becomes a difference of that size between the step sizes of two summation orders, and the chains part there.
 __device__ void hmc_update(ChainState& h, float mh_rate_f) {  // :259-297
   const double mh_rate = (double)mh_rate_f;
   if (h.iteration == h.burnin) {

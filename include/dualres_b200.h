@@ -165,7 +165,7 @@ void dr_chainset_destroy(dr_chainset* cs);
  * where 0 keeps the whole plane in shared memory, 2 x-line kernel with separate y
  * passes), kriging-product blocks per SM, the
  * iteration time measured when the shape was tuned (0 when it was not), and
- * whether the kriging products run on the tensor cores (1; 2 when W^T's chain
+ * whether the kriging products run on the tensor cores (1; 2 when the chain
  * vectors arrive by TMA row gathers) or over groups of rows (0).  At creation the
  * update paths are timed on a scratch chain set of the same shape (with the
  * tensor-core products where available), then the other
