@@ -172,7 +172,7 @@ static void set_pass_attrs() {
   set_smem(k_pass<N, +1, C>, bytes);
   if constexpr (sizeof(C) == 8) {
     set_smem(k_xline<N>, bytes);
-    if constexpr (N <= 256) set_z_attrs<N, 0>();
+    set_z_attrs<N, 0>();
     if constexpr (two_plans(N)) {
       set_z_attrs<N, 1>();
       set_smem(k_xline<N, 1>, bytes);
@@ -223,7 +223,6 @@ template <class C>
 static void set_all_attrs() {
   set_pass_attrs<2, C>(); set_pass_attrs<4, C>(); set_pass_attrs<8, C>(); set_pass_attrs<16, C>();
   set_pass_attrs<32, C>(); set_pass_attrs<64, C>(); set_pass_attrs<128, C>(); set_pass_attrs<256, C>();
-  if constexpr (sizeof(C) == 8) set_pass_attrs<512, C>();
 }
 
 static DeviceTables& device_tables(int dev) {
@@ -243,7 +242,7 @@ static DeviceTables& device_tables(int dev) {
   }
   std::vector<float2> hf(TW_TOTAL);
   std::vector<double2> hd(TW_TOTAL);
-  for (int N = 2; N <= 512; N <<= 1)
+  for (int N = 2; N <= MAX_AXIS; N <<= 1)
     for (int m = 0; m < N; m++) {
       const double a = -2.0 * M_PI * (double)m / (double)N;
       hd[tw_offset(N) + m] = make_double2(std::cos(a), std::sin(a));
@@ -323,12 +322,6 @@ static void launch_pass(int n, int dir, const PassArgs& a, const DevChains& ch, 
     case 64: launch_pass_n<64, C>(dir, a, ch, tw, nch, s); break;
     case 128: launch_pass_n<128, C>(dir, a, ch, tw, nch, s); break;
     case 256: launch_pass_n<256, C>(dir, a, ch, tw, nch, s); break;
-    case 512:
-      if constexpr (sizeof(C) == 8) {
-        launch_pass_n<512, C>(dir, a, ch, tw, nch, s);
-        break;
-      }
-      [[fallthrough]];
     default: throw Error(DR_ERR_UNSUPPORTED, "FFT length not supported: " + std::to_string(n));
   }
 }
@@ -1028,7 +1021,6 @@ static void launch_xline(Chainset* S, int step, int flags) {
       if (S->dc.fftplan & FP_XLINE) launch_k(k_xline<256, 1>, grid, 256, smem, S->stream, v, S->dc, step, flags, tw);
       else launch_k(k_xline<256>, grid, 256, smem, S->stream, v, S->dc, step, flags, tw);
       break;
-    case 512: launch_k(k_xline<512>, grid, 512, smem, S->stream, v, S->dc, step, flags, tw); break;
     default: throw Error(DR_ERR_UNSUPPORTED, "E0 not supported");
   }
   CK_LAUNCH();
@@ -1534,8 +1526,10 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
     ch.nb_w = tc_finish_blocks(V->tc_w.T);
     ch.nb_wt = tc_finish_blocks(V->tc_wt.T);
     S->tc_partial = S->alloc<float>((size_t)std::max(V->tc_max_segs, 1) * S->tc_N * TC_M, false);
-    // TMA row gathers from 32 chains (rows of 128 bytes): 64 chains on a 32^3 volume W 23.7 / W^T 20.3 us against 25.0 /
-    // 20.9 with the threads' own loads, 16 chains on 64x64x48 61.3 / 46.2 against 58.0 / 45.2
+    // TMA row gathers where a product has 32 columns or more, from 20 chains (16-byte rows).  W / W^T on 32^3: 20 chains 21.1 /
+    // 16.7 us, 21.9 / 16.9 with the threads' own loads; 64 chains 23.5 / 19.8, 24.5 / 20.3.  On 64x64x48, where the row groups
+    // are the faster below 32 chains (18 chains 69 / 51): 20 chains 82.5 / 61.2, 78.7 / 57.3; 36 chains 87.7 / 72.4, 90.2 /
+    // 72.2; with 16 columns (16 chains) 61.3 / 46.2, 58.0 / 45.2
     const char* tg = std::getenv("DRB_TC_TMA_GATHER");
     S->tc_tg = !(tg && std::string(tg) == "0") && S->tc_N >= 32 && encode_row_map(&S->tc_map_wt, ch.rs, ch.Cp, (long long)v.n_s, S->tc_N) &&
                encode_row_map(&S->tc_map_w, ch.muD, ch.Cp, 2LL * v.n_h, S->tc_N);
@@ -1548,8 +1542,8 @@ static void chainset_build(Chainset* S, Volume* V, int C, const dr_hmc_opts* o, 
       ch.nb_wt = std::max(1, std::min(cdiv_i((long long)v.n_h * C, ROWP_NT), S->sms * 8));
     }
   }
-  // k_momentum's row groups, at most four blocks per SM taking them in turn
-  ch.nb_g = std::min(cdiv_i((long long)v.EZ * v.E1, MOM_ITEMS / v.E0), 592);
+  // k_momentum's row groups; a chain's blocks, at most four per SM, take them in turn
+  ch.nb_g = std::min(cdiv_i((long long)v.EZ * v.E1, MOM_ITEMS / v.E0), 4 * S->sms);
   ch.maxblk = std::max(ch.nb_x + ch.nb_g, std::max(ch.nb_w, ch.nb_wt));
   ch.part = S->alloc<double>((size_t)C * NSLOT * ch.maxblk);
   ch.st = S->alloc<ChainState>(C);

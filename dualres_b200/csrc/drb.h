@@ -7,7 +7,7 @@
 namespace drb {
 
 // Largest FFT length per axis handled by the shared-memory kernels.
-constexpr int MAX_AXIS = 512;
+constexpr int MAX_AXIS = 256;
 // Lines per tile in the pass kernels.
 constexpr int TILE_LINES = 32;
 

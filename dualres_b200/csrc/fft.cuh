@@ -1,4 +1,4 @@
-// Shared-memory Stockham FFT for power-of-two lengths 2..512.
+// Shared-memory Stockham FFT for power-of-two lengths 2..256.
 //
 // A tile of `nlines` independent lines sits in shared memory; element i of
 // line l lives at sm[l * ls + i * es].  Each stage of radix R splits every
@@ -177,10 +177,10 @@ __device__ __forceinline__ void warp_stage(C* L, int es, int b, bool on, const C
 // Largest butterfly count per line over the stages of the plan for N.
 template <int N>
 __host__ __device__ constexpr int plan_nbmax() {
-  return N <= 16 ? 1 : (N == 32 ? 8 : (N == 64 ? 8 : (N == 128 ? 16 : 16)));
+  return N <= 16 ? 1 : 8;
 }
 
-// Warp-synchronous FFT of nlines lines (N <= 256): each warp takes groups of
+// Warp-synchronous FFT of nlines lines (N <= 32): each warp takes groups of
 // 32 / nbmax lines; every stage runs with warp-level synchronisation only.
 // The block synchronises once at the end, so the tile is complete on return.
 template <int N, int DIR, class C>
@@ -194,18 +194,10 @@ __device__ __forceinline__ void fft_smem_warp(C* sm, int ls, int es, int nlines,
     C* L = sm + (on ? line : 0) * ls;
     if constexpr (N <= 16) {
       warp_stage<N, N, 1, DIR, C>(L, es, b, on, tw);
-    } else if constexpr (N == 32) {
+    } else {
+      static_assert(N == 32, "longer lines go through fft_smem or the padded planes");
       warp_stage<32, 8, 1, DIR, C>(L, es, b, on, tw);
       warp_stage<32, 4, 8, DIR, C>(L, es, b, on, tw);
-    } else if constexpr (N == 64) {
-      warp_stage<64, 8, 1, DIR, C>(L, es, b, on, tw);
-      warp_stage<64, 8, 8, DIR, C>(L, es, b, on, tw);
-    } else if constexpr (N == 128) {
-      warp_stage<128, 16, 1, DIR, C>(L, es, b, on, tw);
-      warp_stage<128, 8, 16, DIR, C>(L, es, b, on, tw);
-    } else {
-      warp_stage<256, 16, 1, DIR, C>(L, es, b, on, tw);
-      warp_stage<256, 16, 16, DIR, C>(L, es, b, on, tw);
     }
   }
   __syncthreads();
@@ -245,17 +237,13 @@ __device__ __forceinline__ void fft_smem(C* sm, int ls, int es, int nlines, cons
   } else if constexpr (N == 256) {
     fft_stage<256, 16, 1, DIR, cdiv(16 * MAXLINES, NTHR), C>(sm, ls, es, nlines, tw, tid, NTHR);
     fft_stage<256, 16, 16, DIR, cdiv(16 * MAXLINES, NTHR), C>(sm, ls, es, nlines, tw, tid, NTHR);
-  } else if constexpr (N == 512) {
-    fft_stage<512, 8, 1, DIR, cdiv(64 * MAXLINES, NTHR), C>(sm, ls, es, nlines, tw, tid, NTHR);
-    fft_stage<512, 8, 8, DIR, cdiv(64 * MAXLINES, NTHR), C>(sm, ls, es, nlines, tw, tid, NTHR);
-    fft_stage<512, 8, 64, DIR, cdiv(64 * MAXLINES, NTHR), C>(sm, ls, es, nlines, tw, tid, NTHR);
   }
 }
 
 // Offset of the twiddle table for length N in the concatenated table
-// (lengths 2, 4, ..., 512; entry m of length N is exp(-2 pi i m / N)).
+// (lengths 2, 4, ..., 256; entry m of length N is exp(-2 pi i m / N)).
 __host__ __device__ constexpr int tw_offset(int N) { return N - 2; }
-constexpr int TW_TOTAL = 1022;
+constexpr int TW_TOTAL = 510;
 
 // ----------------------------------------------------------------- padded 2D planes
 // An E x E plane (k_plane_square) stored with one pad slot after every 8 elements along both

@@ -824,7 +824,7 @@ int host_prepare(const dr_volume_desc* d, HostVolume* hv, std::string* err, bool
     int p = 1;
     while (p < 2 * (hv->g[k] - 1)) p <<= 1;
     hv->E[k] = p;
-    if (p > 256) { *err = "dr_volume_create: embedding dimension above 256 is not supported"; return DR_ERR_UNSUPPORTED; }
+    if (p > MAX_AXIS) { *err = "dr_volume_create: embedding dimension above 256 is not supported"; return DR_ERR_UNSUPPORTED; }
   }
   hv->N = (long long)hv->E[0] * hv->E[1] * hv->E[2];
   if (hv->N > (1LL << 30)) { *err = "dr_volume_create: embedding too large"; return DR_ERR_UNSUPPORTED; }

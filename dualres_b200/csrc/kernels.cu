@@ -119,7 +119,7 @@ __device__ double gamma_draw(double shape, double scale, uint64_t seed, uint32_t
 // lines (line = a * B + b) of one chain (blockIdx.y) per block: the y passes of
 // the x-line path, the initial state and the unpruned 3D transforms.
 template <int N> struct PassCfg {
-  static constexpr int NT = N >= 512 ? 512 : 256;
+  static constexpr int NT = 256;
 };
 
 template <int N, int DIR, class C>
@@ -503,13 +503,12 @@ __global__ void k_split(DevVolume v, const float2* __restrict__ u, float2* __res
 //   drift u* += eps q / lambda_m                              (:693-698)
 //   forward x-FFT of u* for the next gradient.
 // Step 0 starts from the momentum that k_momentum drew and adds the initial
-// energies; the
-// last step only kicks and accumulates the final energies (:702-705).
+// energies; the last step only kicks and accumulates the final energies (:702-705).
 template <int E0> struct XCfg {
-  static constexpr int NT = E0 >= 512 ? 512 : 256;
+  static constexpr int NT = 256;
   // blocks per SM the register budget targets: at E0 = 256 the 67.6 KB tile allows three (85 registers, no
   // spills; two at the unconstrained 126 registers), at E0 <= 128 four
-  static constexpr int MINB = E0 >= 512 ? 1 : (E0 == 256 ? 3 : 4);
+  static constexpr int MINB = E0 == 256 ? 3 : 4;
 };
 
 template <int E0, int PLAN = 0>
@@ -695,77 +694,59 @@ __device__ __forceinline__ void plane_update(float2* sm, const DevVolume& v, con
   const bool fixed = (flags & XF_FIXED_MOMENTUM) != 0;
   double pa = 0.0, pb = 0.0;
   // Pairs of x-adjacent points: element pair e sits at li = 2e of the plane (x = 2 (e mod E/2), y = e / (E/2)),
-  // so U, q and 1/lambda are read as float4 / float4 / float2 at index e.  Each thread issues the loads of B pairs
-  // before computing them; with the block's state prefetched into L2 at entry one pair suffices (two pairs were
-  // 154.7 against 151.8 us for a 64^2 plane x 64 chains).  A thread reads and writes only its own elements, which is
-  // why the in-place state buffers may be marked non-aliasing.
+  // so U, q and 1/lambda are read as float4 / float4 / float2 at index e: one pair at a time, the block's state being
+  // prefetched into L2 at entry.  A thread reads and writes only its own elements, which is why the in-place state
+  // buffers may be marked non-aliasing.
   constexpr int TOTAL = E * (E / 2);
-  constexpr int B = 1;
   const float4* __restrict__ gU = reinterpret_cast<const float4*>(srcU);
   const float4* __restrict__ gQ = reinterpret_cast<const float4*>(srcQ);
   const float2* __restrict__ gS = reinterpret_cast<const float2*>(srcS);
   float4* __restrict__ oQ = reinterpret_cast<float4*>(Qc);
   float4* __restrict__ oU = reinterpret_cast<float4*>(Udst);
-  for (int e0 = tid; e0 < TOTAL; e0 += B * NT) {
-    float4 u4v[B], q4v[B];
-    float2 s2v[B];
+  for (int e = tid; e < TOTAL; e += NT) {
+    const float4 u4 = __ldcs(gU + e);
+    const float4 q4 = __ldcs(gQ + e);
+    const float2 s2 = gS[e];
+    const int y = e / (E / 2), x = 2 * (e % (E / 2));
+    const int pi0 = G::at(y, x), pi1 = pi0 + 1;  // x is even: x + 1 is the next slot in either layout
+    float2 uo[2], qo[2];
 #pragma unroll
-    for (int b = 0; b < B; b++) {
-      const int e = e0 + b * NT;
-      if (e < TOTAL) {
-        u4v[b] = __ldcs(gU + e);
-        q4v[b] = __ldcs(gQ + e);
-        s2v[b] = gS[e];
+    for (int m = 0; m < 2; m++) {
+      const float2 u = m == 0 ? make_float2(u4.x, u4.y) : make_float2(u4.z, u4.w);
+      const float s = m == 0 ? s2.x : s2.y;
+      const bool live = s > 0.0f;
+      const float lm = s + sh;
+      float2 q = m == 0 ? make_float2(q4.x, q4.y) : make_float2(q4.z, q4.w);
+      if (first && live) {  // the kinetic energy of a drawn momentum is k_momentum's sum |w|^2
+        if (fixed) pa += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+        pb += (double)(u.x * u.x + u.y * u.y) * (double)s;
       }
-    }
-#pragma unroll
-    for (int b = 0; b < B; b++) {
-      const int e = e0 + b * NT;
-      if (e >= TOTAL) continue;
-      const int y = e / (E / 2), x = 2 * (e % (E / 2));
-      const float4 u4 = u4v[b];
-      const float2 s2 = s2v[b];
-      const float4 q4 = q4v[b];
-      const int pi0 = G::at(y, x), pi1 = pi0 + 1;  // x is even: x + 1 is the next slot in either layout
-      float2 uo[2], qo[2];
-#pragma unroll
-      for (int m = 0; m < 2; m++) {
-        const float2 u = m == 0 ? make_float2(u4.x, u4.y) : make_float2(u4.z, u4.w);
-        const float s = m == 0 ? s2.x : s2.y;
-        const bool live = s > 0.0f;
-        const float lm = s + sh;
-        float2 q = m == 0 ? make_float2(q4.x, q4.y) : make_float2(q4.z, q4.w);
-        if (first && live) {  // the kinetic energy of a drawn momentum is k_momentum's sum |w|^2
-          if (fixed) pa += (double)(q.x * q.x + q.y * q.y) / (double)lm;
-          pb += (double)(u.x * u.x + u.y * u.y) * (double)s;
-        }
-        const int pi = m == 0 ? pi0 : pi1;
-        const float2 g = sm[pi];
-        float2 gt = g;
-        if (live) {
-          gt.x = fmaf(-u.x, s, g.x);
-          gt.y = fmaf(-u.y, s, g.y);
-        }
-        q.x = fmaf(keps, gt.x, q.x);
-        q.y = fmaf(keps, gt.y, q.y);
-        float2 un = u;
-        if (last) {
-          if (live && !first) {  // first and last: an evaluation step, energies at mu only
-            pa += (double)(u.x * u.x + u.y * u.y) * (double)s;
-            pb += (double)(q.x * q.x + q.y * q.y) / (double)lm;
-          }
-        } else if (live) {
-          const float f = eps / lm;
-          un.x = fmaf(f, q.x, u.x);
-          un.y = fmaf(f, q.y, u.y);
-        }
-        uo[m] = un;
-        qo[m] = q;
-        sm[pi] = un;
+      const int pi = m == 0 ? pi0 : pi1;
+      const float2 g = sm[pi];
+      float2 gt = g;
+      if (live) {
+        gt.x = fmaf(-u.x, s, g.x);
+        gt.y = fmaf(-u.y, s, g.y);
       }
-      if (write_q) __stcs(oQ + e, make_float4(qo[0].x, qo[0].y, qo[1].x, qo[1].y));
-      if (!last) __stcs(oU + e, make_float4(uo[0].x, uo[0].y, uo[1].x, uo[1].y));
+      q.x = fmaf(keps, gt.x, q.x);
+      q.y = fmaf(keps, gt.y, q.y);
+      float2 un = u;
+      if (last) {
+        if (live && !first) {  // first and last: an evaluation step, energies at mu only
+          pa += (double)(u.x * u.x + u.y * u.y) * (double)s;
+          pb += (double)(q.x * q.x + q.y * q.y) / (double)lm;
+        }
+      } else if (live) {
+        const float f = eps / lm;
+        un.x = fmaf(f, q.x, u.x);
+        un.y = fmaf(f, q.y, u.y);
+      }
+      uo[m] = un;
+      qo[m] = q;
+      sm[pi] = un;
     }
+    if (write_q) __stcs(oQ + e, make_float4(qo[0].x, qo[0].y, qo[1].x, qo[1].y));
+    if (!last) __stcs(oU + e, make_float4(uo[0].x, uo[0].y, uo[1].x, uo[1].y));
   }
   const double wt = plane_weight(z, v.E2);
   pa_out = wt * pa;
@@ -842,8 +823,8 @@ __global__ void __launch_bounds__(SquareCfg<WIDE>::NT, SquareCfg<WIDE>::MINB) k_
   const float* Sg = v.sinv + (long long)z * E * E;
   float2* T = ch.T2 + (long long)c * ch.t2_stride + (long long)z * by * bx;
   // the twiddles of length E in shared memory: the row and column stages load a lane's twiddles again for every
-  // line, and as global loads (L1 hits) they were most of the kernel's load instructions (146.8 -> 140.9 us for
-  // 64^2 planes x 64 chains)
+  // line, and as global loads (L1 hits) they were most of the kernel's load instructions (4 % of its time on the full
+  // spectrum)
   __shared__ float2 twE[E];
   for (int i = tid; i < E; i += NT) twE[i] = tw[tw_offset(E) + i];
   if ((flags & XF_L2_PREFETCH) && tid == 0) {
