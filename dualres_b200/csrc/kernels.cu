@@ -23,7 +23,8 @@
 // planes 0 < kz < E2/2 by two (plane_weight).  Measured against the full complex
 // state (64 chains on a 64^3 embedding): update 139 -> 73 us, forward / inverse z
 // pass 20.4 / 18.1 -> 10.6 / 10.1 us, an iteration 6.1 -> 4.1 ms; 16 chains on
-// 128^3: update 458 -> 252 us, z 38 / 34 -> 16 / 17 us.
+// 128^3: update 458 -> 252 us, z 38 / 34 -> 16 / 17 us (since then the plane kernels below:
+// 68 and 177 us).
 #include "common.cuh"
 #include "drb.h"
 #include "fft.cuh"
@@ -856,8 +857,8 @@ __global__ void __launch_bounds__(SquareCfg<WIDE>::NT, SquareCfg<WIDE>::MINB) k_
 // Measured: 16 chains on 128^3 177 us (whole plane in shared memory, 512
 // threads: 246; x-line kernel with its y passes 190 + 61); 12 chains on 128x64x32 18.7 us
 // (x-line 17.5 + 8.2); 64 chains on 64^3 87 us (k_plane_square 68). It is bound
-// by the L1 pipe (77 %): bank conflicts of the exchanges and the state's runs of
-// 16 LN bytes.  Loading a row's whole state before its inverse transform was slower
+// by latency: its registers leave 16 warps to an SM, which wait on the state (L1 pipe
+// 48 %, DRAM 39 %, 3.2 TB/s).  Loading a row's whole state before its inverse transform was slower
 // (128^3: 222 us: it spills at 128 registers).
 // WIDE: 512 threads with all the registers, for chain sets of at most a plane per SM (4 chains on 128x128x64: 21.4 us,
 // 27.9 with the narrow blocks).

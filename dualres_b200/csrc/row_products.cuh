@@ -25,8 +25,9 @@
 // memory on large volumes) and the chain vectors (L1 / L2).  Measured (W / W^T,
 // us; before: CSR rows): 1 chain, 32^3 volume 5.8 / 5.7 (7.8 / 7.9); 2 chains,
 // 80x80x64, 510 MB of entries 56 / 47, 4.9 TB/s (134 / 160); 12 chains, 43x23x17
-// 9.0 / 10.1 (23 / 20); 16 chains, 64x64x48 29.5 / 29 (tensor-core tiles 58 / 45,
-// whose dense blob is 8 times the entries there).  Tried: groups of single rows
+// 9.0 / 10.1 (23 / 20); 16 chains, 64x64x48 29.5 / 29 launched back to back and 35 /
+// 33 inside an iteration (tensor-core tiles 58 / 45, whose dense blob is 8 times the
+// entries there).  Tried: groups of single rows
 // (W 78 us on 80x80x64), entries streamed through a shared-memory ring by
 // cp.async (88 / 71 us: the ring takes the L1 that the chain vectors hit).
 #pragma once
